@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(kAdjThreads, 6) adjointKernel(const __grid_con
     const float4 wsi = doSlow ? a.wS[iatom] : make_float4(0.f, 0.f, 0.f, 0.f);
     float gix = 0.f, giy = 0.f, giz = 0.f, giq = 0.f;
     for (int jt = tl.jtileStart; jt <= tl.jtileEnd; ++jt) {
-      const unsigned mask = a.tileExcls[jt].excl[lane];
+      // from block order to rows (bit j of lane i), then bit t <-> j = (lane + t) & 31
+      const unsigned rowMask = blockOrder(a.tileExcls[jt].excl[lane], lane);
+      const unsigned mask = __funnelshift_r(rowMask, rowMask, lane);
       unsigned stepMask = __reduce_or_sync(0xffffffffu, mask);
       if (!stepMask) continue;
       const int jstart = a.tileJatomStart[jt];

@@ -86,6 +86,7 @@ struct nbk_context {
   nbk_params prm{};
   NbkConst c{};
   NbkConst64 c64{};
+  PackedConst pk{};
   int ljDim = 0;
   DBuf<float2> ljTable, ljExclTable;
   DBuf<double2> slowTable;  // FP64 phi_s rows (buildSlowTable)
@@ -184,8 +185,8 @@ struct nbk_context {
 namespace {
 // Default launch shape of the force kernel: 4 CTAs per SM (a 128-register
 // cap), one warp per tile list; measured fastest at 92k atoms for the energy
-// and slow-force evaluations under flushed-L2 conditions (0.405 vs 0.411 ms
-// at 5 CTAs per SM for energy + virial + slow).
+// and slow-force evaluations (steady steps, fast + slow forces 280 us against
+// 281 at 5 and 290 at 6 CTAs per SM; with energies and virials 494, 502, 510).
 constexpr int kDefaultMinBlocks = 4;
 constexpr int kMaxTimed = 4096;
 
@@ -251,6 +252,7 @@ ForceArgs refinedForceArgs(nbk_context* h, float cutoff2) {
   a.latc = h->latc;
   a.c = h->c;
   a.c.cutoff2 = cutoff2;
+  a.pk = h->pk;
   a.force = h->force.p;
   a.stride = h->atomStorageSize;
   a.acc = h->acc.p;
@@ -348,6 +350,7 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   h->prm.ljA = h->prm.ljB = h->prm.ljA14 = h->prm.ljB14 = nullptr;
   h->ljDim = p->vdwTableDim;
   makeConstants(*p, p->vdwTableDim, h->c, h->c64);
+  makePacked(h->c64, h->pk);
   for (int k = 0; k < 32; ++k) {
     h->tuneMinBlocks[k] = kDefaultMinBlocks;
     h->tuneSplitLog2[k] = 0;
@@ -865,7 +868,21 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
   if (jatom && cnt[1])
     NBK_CUDA(cudaMemcpy(jatom, h->jatom2.p, sizeof(int) * cnt[1], cudaMemcpyDeviceToHost), "export");
   if (excl && cnt[1])
+  {
     NBK_CUDA(cudaMemcpy(excl, h->excl2.p, sizeof(nbk_tile_excl) * cnt[1], cudaMemcpyDeviceToHost), "export");
+    // from block order to the interface's: bit t of lane i <-> j = (i + t) & 31
+    for (int k = 0; k < cnt[1]; ++k) {
+      unsigned w[32];
+      std::memcpy(w, excl[k].excl, sizeof(w));
+      for (int i = 0; i < 32; ++i) {
+        unsigned row = 0;
+        for (int lj = 0; lj < 4; ++lj)
+          row |= ((w[8 * lj + (i & 7)] >> (i >> 3)) & 0x11111111u) << lj;
+        if (i & 4) row = ((row >> 4) & 0x0f0f0f0fu) | ((row & 0x0f0f0f0fu) << 4);
+        excl[k].excl[i] = (row >> i) | (i ? row << (32 - i) : 0u);
+      }
+    }
+  }
   return NBK_OK;
 }
 
@@ -955,7 +972,7 @@ NBK_API int nbk_set_replicas(nbk_handle h, int numReplicas, const int* repOfComp
   std::vector<float2> t((size_t)numReplicas * d2), te((size_t)numReplicas * d2);
   const double sc = h->prm.scaling;
   for (size_t k = 0; k < t.size(); ++k) {
-    t[k] = make_float2((float)(ljA[k] * sc), (float)(ljB[k] * sc));
+    t[k] = make_float2((float)(ljA[k] * sc), -(float)(ljB[k] * sc));  // (A, -B)
     const double a14 = ljA14 ? ljA14[k] : ljA[k], b14 = ljB14 ? ljB14[k] : ljB[k];
     te[k] = make_float2((float)((a14 - ljA[k]) * sc), (float)((b14 - ljB[k]) * sc));
   }

@@ -34,11 +34,8 @@ void makeConstants(const nbk_params& p, int ljDim, NbkConst& c, NbkConst64& k) {
   c.beta = (float)p.ewaldcof;
   c.beta2Pi = (float)(2.0 * p.ewaldcof / std::sqrt(M_PI));
   c.one14 = (float)(1.0 - p.scale14);
-  c.pBeta = (float)(kErfcP * p.ewaldcof);
-  c.gaussK = (float)(-p.ewaldcof * p.ewaldcof / std::log(2.0));
   c.ljDim = ljDim;
   c.switching = sw ? 1 : 0;
-  c.s0 = sw ? 0.0f : 1.0f;
   c.hAd = 1.5 / rc;
   c.hBd = -0.5 / (rc * rc2);
   c.betad = p.ewaldcof;
@@ -55,6 +52,21 @@ void makeConstants(const nbk_params& p, int ljDim, NbkConst& c, NbkConst64& k) {
   k.beta2Pi = 2.0 * p.ewaldcof / std::sqrt(M_PI);
   k.one14 = 1.0 - p.scale14;
   k.switching = sw ? 1 : 0;
+}
+
+// The packed pair math's constants (formulas at PackedConst).
+void makePacked(const NbkConst64& k, PackedConst& c) {
+  auto pair = [](double v) { return make_float2((float)v, (float)v); };
+  const double D = k.switching ? k.rc2 - k.rs2 : 1.0, c1 = 1.0 / (D * D * D);
+  c.dA = pair(-12.0 * c1 * D);
+  c.dB = pair(12.0 * c1);
+  c.hA = pair(-6.0 * c1 * D);
+  c.rc3inv = pair(k.rc3inv);
+  c.nBeta2Pi = pair(-k.beta2Pi);
+  c.rc2 = k.switching ? (float)k.rc2 : 1.0e30f;
+  c.dMax = (float)D;
+  c.pBeta = (float)(kErfcP * k.beta);
+  c.gaussK = (float)(-k.beta * k.beta / std::log(2.0));
 }
 
 namespace {

@@ -4,12 +4,13 @@
 // forceKernel: one warp owns one tile list (32 i atoms of one patch against
 // the j tiles of a compute's partner patch), as CudaComputeNonbondedKernel's
 // nonbondedForceKernel does (src/CudaComputeNonbondedKernel.cu:629-1644), but:
-//   - two pair steps per iteration run through sm_100's packed FP32
-//     instructions; j forces ride in registers and rotate with a shuffle, so
-//     the inner loop touches shared memory only for the j-tile loads;
-//   - steps whose bit is clear in every lane's mask are skipped warp-uniformly;
+//   - a tile is taken as 16 blocks of 8 x 8 atoms, one pass of the warp each
+//     (two pairs per lane through sm_100's packed FP32 instructions); i and j
+//     forces ride in registers and are reduced over lanes per row of blocks
+//     and per group of tiles;
+//   - blocks without listed pairs are skipped warp-uniformly;
 //   - the lists it reads are already refined (TileExcl masks from
-//     refineKernel); a pairlist step refines, compacts, then runs this kernel;
+//     refineKernel, in block order); a pairlist step refines, compacts, then runs this kernel;
 //   - per-tile FP32 partial forces are folded into 64-bit fixed point with
 //     integer atomics, so the summed forces do not depend on the order in
 //     which lists run; the LJ energy is summed in FP32 per group of tiles and
@@ -184,13 +185,14 @@ __device__ __forceinline__ void precisePair(const PairTerms& u, const SlowTable&
   }
 }
 
-// The FP64 pair terms of the pair (i, j = (i + t) & 31) from the warp's atoms
-// in shared memory; qq = 0 (exact zeros) when the lane has no pair left and
+// The FP64 pair terms of the pair of owner lane l and bit t (block order) from
+// the warp's atoms in shared memory; qq = 0 (exact zeros) when the lane has no pair left and
 // repeats its last one, a real interacting pair (so its distance is not 0).
-__device__ __forceinline__ void pairTerms(const Atoms64& A, const int i, const int t,
+__device__ __forceinline__ void pairTerms(const Atoms64& A, const int l, const int t,
                                           const bool valid, PairTerms& u) {
+  const int i = ((t & 3) << 3) | (l & 7), j = ((t & 28) ^ (l & 4)) | (l >> 3);
   const double2 ia = A.ixy[i], ib = A.izq[i];
-  const float4 jb = A.j[(i + t) & 31];
+  const float4 jb = A.j[j];
   u.dx = (double)jb.x - ia.x;
   u.dy = (double)jb.y - ia.y;
   u.dz = (double)jb.z - ib.x;
@@ -236,10 +238,10 @@ __device__ __forceinline__ void walkNext(PairWalk& s, const bool valid, const un
   }
 }
 
-// The precise pass of one tile. live (per lane): bit t set when the pair
-// (i = lane, j = (lane + t) & 31) is an interacting pair (mask bit set and
-// FP32 r^2 below the cutoff, the classification the FP32 math used). The
-// tile's `total` interacting pairs, in lane-major order (by i, then t), are
+// The precise pass of one tile. live (per lane): bit t set when the pair that
+// lane and bit stand for in block order is an interacting pair (mask bit set
+// and FP32 r^2 below the cutoff, the classification the FP32 math used). The
+// tile's `total` interacting pairs, in lane-major order (by lane, then t), are
 // split into 32 contiguous ranges of m = ceil(total / 32): lane k takes pairs
 // k m .. k m + m - 1 (the last lanes fewer or none). A lane finds the owner
 // of its first pair by a binary search over the lanes' inclusive counts
@@ -339,9 +341,37 @@ __device__ __forceinline__ void reduceGroup(const int lane, LaneSums& L, long lo
   L = LaneSums{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 }
 
+// One reduction step over a pair of lanes (l and l ^ o): every lane keeps one
+// of its two values, the lane whose bit o is clear the first, the other the
+// second, and adds its partner's share of the one it keeps.
+__device__ __forceinline__ float keepHalf(const float first, const float second, const bool bit,
+                                          const int o) {
+  const float send = bit ? first : second;
+  const float keep = bit ? second : first;
+  return keep + __shfl_xor_sync(0xffffffffu, send, o);
+}
+
+// Block order: a 32 x 32 tile is 16 blocks of 8 i atoms by 8 j atoms. Lane
+// l = 8 lj + li (li = l & 7, lj = l >> 3) takes, of block (I, J), the pairs of
+// i = 8 I + li with j = 8 J + lj and j + 4 (elements x and y of the packed
+// math; the other way round in the lanes with bit 2 set), so a block is one pass of the packed loop with every lane
+// busy, its j atoms' sums stay in registers over the blocks of a row (the same
+// J) and its i atoms' over a group of tiles: the loop has no shuffle. The mask
+// words hold bit 8 J + 4 e + I of element e (blockOrder; TileExcl rows are put into this
+// order by the refinement and back by the export).
+//
+// What bounds it: issue slots and the FMA pipe, as before, but on far fewer
+// passes. Blocks of 8 x 8 atoms are compact (the atom order bisects down to 8),
+// so a pass holds 28.5 interacting pairs of 64 (20k mixed system; 255,843
+// passes) where the diagonals j = (l + t) & 31 of the tile held 17.4
+// (419,488), and the diagonals' rotation of the j sums (12 shuffles a pass)
+// becomes one reduction per row of blocks. Steady steps of the 92,224-atom
+// mixed system: fast + slow forces 392 -> 290 us, fast forces 279 -> 198 us,
+// with energies and virials 601 -> 507 us (of which the precise kernel is 200);
+// 210 M warp instructions for fast + slow forces.
+//
 // MINB: CTAs per SM the register budget is cut for (4, 5 or 6 -> 128, 96 or
-// 80 registers; the packed loop holds two pairs' state, and 5 is the untuned
-// default); a.splitLog2: each list's j tiles are shared by 2^splitLog2
+// 80 registers); a.splitLog2: each list's j tiles are shared by 2^splitLog2
 // work items (warps), contiguous parts of equal tile count. Both are launch
 // choices of the autotuner; results do not depend on them (fixed-point sums
 // per tile group).
@@ -351,16 +381,20 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
   // the live words feed the precise kernel, which runs on energy evaluations
   // and on virial evaluations with slow forces (it forms the slow virial)
   constexpr bool kLive = doEnergy || (doVirial && doSlow);
-  extern __shared__ __align__(16) float2 s_lj[];  // [ljDim*ljDim] (single system)
-  // the j tile as five rows (x, y, z, q, type bits) of 64 entries; entry m
-  // holds the values of atoms m & 31 and (m & 31) ^ 16, so that the two
-  // packed elements of iteration k, j = (lane + k) & 31 and j ^ 16, come from
-  // one 8-byte load at the fixed offset lane + k
-  __shared__ float2 s_jt[kForceWarps][5][2 * kWarp];
+  constexpr int kNC = doSlow ? 6 : 3;  // force components: fast x y z, slow x y z
+  extern __shared__ __align__(16) float2 s_lj[];  // [ljDim*ljDim] (A, -B) (single system)
+  // the list's i atoms, shifted: (-x, -x, -y, -y), then (-z, -z, q, byte
+  // offset of the type's LJ row)
+  __shared__ float4 s_i[kForceWarps][2][kWarp];
+  // the j tile by pairs (j, j + 4) of a row's lanes: entry 4 J + lj holds
+  // (x, x', y, y'), (z, z', q, q') and (type, type') as byte offsets in an LJ
+  // row; the second copy, for the lanes with bit 2 set, holds j + 4 first
+  __shared__ float4 s_j[kForceWarps][2][2][16];
+  __shared__ float2 s_jt[kForceWarps][2][16];
   // each lane's i force of the current list part in fixed point, folded in
   // at the end of every tile group, so that the sums do not depend on how a
   // list's tiles are split among warps
-  __shared__ long long s_fi[kForceWarps][6][kWarp];
+  __shared__ long long s_fi[kForceWarps][kNC][kWarp];
   // each lane's LJ energy of the list part in fixed point (s_ev) and of the
   // current tile group in FP32 (s_evg), and the warp's fixed-point LJ total
   // (s_evw, lane 0), kept in shared memory rather than in registers the pair
@@ -371,10 +405,15 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
 
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
+  const int li = lane & 7, lj = lane >> 3;
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
+  const unsigned adrI = sharedAddr(&s_i[wib][0][li]), adrJ = sharedAddr(&s_j[wib][b2][0][lj]),
+                 adrT = sharedAddr(&s_jt[wib][b2][lj]), adrLJ = sharedAddr(s_lj);
   const NbkConst& c = a.c;
   const int dim = c.ljDim;
   if (!doBatch) {
-    for (int k = threadIdx.x; k < dim * dim; k += blockDim.x) s_lj[k] = a.ljTable[k];
+    for (int k = threadIdx.x; k < dim * dim; k += blockDim.x)
+      s_lj[k] = make_float2(a.ljTable[k].x, -a.ljTable[k].y);
     __syncthreads();
   }
 
@@ -382,7 +421,7 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
 
   long long accVdw = 0;  // lane 0: LJ energy to flush (batched replica change)
 #pragma unroll
-  for (int q = 0; q < 6; ++q) s_fi[wib][q][lane] = 0;
+  for (int q = 0; q < kNC; ++q) s_fi[wib][q][lane] = 0;
   s_ev[wib][lane] = 0;
   s_evg[wib][lane] = 0.f;
   if (lane == 0) s_evw[wib] = 0;
@@ -405,7 +444,7 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
     const int jtLast = min(tl.jtileEnd, jtFirst + chunk - 1);
     if (jtLast < jtFirst) continue;  // this part has no tiles
     float3 la = a.lata, lb = a.latb, lc = a.latc;
-    const float2* ljRow = nullptr;  // batched: this replica's LJ table (global)
+    const char* ljRow = nullptr;  // batched: this replica's LJ table (global)
     if (doBatch) {
       const int rep = __ldg(&a.compRep[tl.icompute]);
       if (rep != curRep) {
@@ -419,22 +458,27 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
       la = a.repLat[3 * rep];
       lb = a.repLat[3 * rep + 1];
       lc = a.repLat[3 * rep + 2];
-      ljRow = a.repLJ + (size_t)rep * dim * dim;
+      ljRow = reinterpret_cast<const char*>(a.repLJ + (size_t)rep * dim * dim);
     }
     const float3 off = make_float3(tl.offsetXYZ.x, tl.offsetXYZ.y, tl.offsetXYZ.z);
     const float3 sh = shiftOf(off, la, lb, lc);
     const bool zeroShift = !(dist2(sh.x, sh.y, sh.z) > 0.0f);
 
     const int iatom = tl.iatomStart + lane;
-    float4 xi = a.xyzq[iatom];
-    xi.x = __fadd_rn(xi.x, sh.x);
-    xi.y = __fadd_rn(xi.y, sh.y);
-    xi.z = __fadd_rn(xi.z, sh.z);
-    const int ti = a.vdwTypes[iatom] * dim;
+    {
+      const float4 xi = a.xyzq[iatom];
+      const float x = -__fadd_rn(xi.x, sh.x), y = -__fadd_rn(xi.y, sh.y),
+                  z = -__fadd_rn(xi.z, sh.z);
+      s_i[wib][0][lane] = make_float4(x, x, y, y);
+      s_i[wib][1][lane] = make_float4(z, z, xi.w, __int_as_float(a.vdwTypes[iatom] * dim * 8));
+    }
 
-    // this tile group's two partial i sums per component
-    float2 fix2 = f2(0.f), fiy2 = f2(0.f), fiz2 = f2(0.f);
-    float2 fisx2 = f2(0.f), fisy2 = f2(0.f), fisz2 = f2(0.f);
+    // this tile group's partial sums of the lane's four i atoms (8 I + li)
+    float fi[4][kNC];
+#pragma unroll
+    for (int I = 0; I < 4; ++I)
+#pragma unroll
+      for (int q = 0; q < kNC; ++q) fi[I][q] = 0.f;
 
     // the next tile's mask word and j atom are loaded while the current tile
     // is computed; the j-tile starts come 32 at a time (lane t holds tile
@@ -455,8 +499,21 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
       }
       const int jstart = __shfl_sync(0xffffffffu, jsBlock, tb);
       const unsigned mask = maskNext;
-      const float4 xj = xjNext;
-      const float tyj = __int_as_float(tyNext);
+      {
+        // atom j = lane of the tile: entry 4 (j >> 3) + (j & 3), element (j >> 2) & 1
+        const int m = (lane >> 3) * 4 + (lane & 3), e = (lane >> 2) & 1;
+#pragma unroll
+        for (int copy = 0; copy < 2; ++copy) {
+          const int ec = copy ? 1 - e : e;
+          float* pa = reinterpret_cast<float*>(&s_j[wib][copy][0][m]) + ec;
+          float* pb = reinterpret_cast<float*>(&s_j[wib][copy][1][m]) + ec;
+          pa[0] = xjNext.x;
+          pa[2] = xjNext.y;
+          pb[0] = xjNext.z;
+          pb[2] = xjNext.w;
+          reinterpret_cast<int*>(&s_jt[wib][copy][m])[ec] = tyNext * 8;
+        }
+      }
       if (jt < jtLast && tb < 31) {
         const int js1 = __shfl_sync(0xffffffffu, jsBlock, tb + 1);
         maskNext = a.tileExcls[jt + 1].excl[lane];
@@ -464,114 +521,119 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
         tyNext = a.vdwTypes[js1 + lane];
       }
       const unsigned stepMask = __reduce_or_sync(0xffffffffu, mask);
-      unsigned live = 0;  // interacting pairs of this lane, TileExcl bit order
-      if (stepMask != 0) {
-        // entry m holds (atom m & 31, atom (m & 31) ^ 16): one 8-byte load
-        // gives both packed elements of an iteration
-        const float2 ex = make_float2(xj.x, __shfl_xor_sync(0xffffffffu, xj.x, 16));
-        const float2 ey = make_float2(xj.y, __shfl_xor_sync(0xffffffffu, xj.y, 16));
-        const float2 ez = make_float2(xj.z, __shfl_xor_sync(0xffffffffu, xj.z, 16));
-        const float2 eq = make_float2(xj.w, __shfl_xor_sync(0xffffffffu, xj.w, 16));
-        const float2 et = make_float2(tyj, __shfl_xor_sync(0xffffffffu, tyj, 16));
-        s_jt[wib][0][lane] = s_jt[wib][0][lane + kWarp] = ex;
-        s_jt[wib][1][lane] = s_jt[wib][1][lane + kWarp] = ey;
-        s_jt[wib][2][lane] = s_jt[wib][2][lane + kWarp] = ez;
-        s_jt[wib][3][lane] = s_jt[wib][3][lane + kWarp] = eq;
-        s_jt[wib][4][lane] = s_jt[wib][4][lane + kWarp] = et;
-        __syncwarp();
-
-        // Iteration k takes steps k and k+16 together through the packed
-        // FP32 math (element x = step k, element y = step k+16); iterations
-        // whose two steps are clear in every lane are skipped. j forces keep
-        // two accumulator sets: P follows step k, Q step k+16, so both rotate
-        // by the same amount; they are folded at the end of the tile.
-        float2 PQx = f2(0.f), PQy = f2(0.f), PQz = f2(0.f);     // (P, Q) fast
-        float2 PQsx = f2(0.f), PQsy = f2(0.f), PQsz = f2(0.f);  // (P, Q) slow
-        float2 eV2 = f2(0.f);
-        const float2 nXi = f2(-xi.x), nYi = f2(-xi.y), nZi = f2(-xi.z);
-        int kLast = 0;
-        unsigned mk = mask;  // bit k of the mask moved to bit 0 (and k+16 to 16)
-#pragma unroll 2
-        for (int k = 0; k < 16; ++k, mk >>= 1) {
-          if (!((stepMask >> k) & 0x10001u)) continue;  // warp-uniform
-          // element x: j = (lane + k) & 31, element y: j ^ 16
-          const float2* pA = &s_jt[wib][0][lane + k];
-          const float2 X = pA[0];
-          const float2 Y = pA[64];
-          const float2 Z = pA[128];
-          const float2 DX = add2(X, nXi), DY = add2(Y, nYi), DZ = add2(Z, nZi);
+      __syncwarp();
+      unsigned live = 0;  // interacting pairs of this lane, block order
+      float2 eV2 = f2(0.f);
+      // live rows, in order; the j sums of a row wait for a partner row (and,
+      // without slow forces, a pair of rows for a partner pair), so that every
+      // lane ends up with one j atom of its own
+      float held[3], held2[3];
+      int Jheld = 0, Jheld2 = 0, rows = 0;
+      unsigned todo = stepMask;
+#pragma unroll 1
+      while (todo) {  // warp-uniform
+        const int J8 = (__ffs(todo) - 1) & 24;  // 8 J
+        const unsigned rowAny = (todo >> J8) & 0xffu;
+        todo &= ~(0xffu << J8);
+        const unsigned mrow = mask >> J8;
+        const float4 ja = ldShared4(adrJ + J8 * 8), jb = ldShared4(adrJ + 256 + J8 * 8);
+        const float2 tj = ldShared2(adrT + J8 * 4);
+        const float2 X = make_float2(ja.x, ja.y), Y = make_float2(ja.z, ja.w),
+                     Z = make_float2(jb.x, jb.y);
+        float2 fj[kNC];
+#pragma unroll
+        for (int q = 0; q < kNC; ++q) fj[q] = f2(0.f);
+        unsigned liveRow = 0;
+#pragma unroll
+        for (int I = 0; I < 4; ++I) {
+          if (!(rowAny & (0x11u << I))) continue;  // warp-uniform
+          const float4 ia = ldShared4(adrI + 128 * I), ib = ldShared4(adrI + 512 + 128 * I);
+          const float2 DX = add2(X, make_float2(ia.x, ia.y)),
+                       DY = add2(Y, make_float2(ia.z, ia.w)),
+                       DZ = add2(Z, make_float2(ib.x, ib.y));
           const float2 R2 = fma2(DZ, DZ, fma2(DX, DX, mul2(DY, DY)));  // dist2's order
-          const bool aA = (mk & 1u) && (R2.x < c.cutoff2);
-          const bool aB = (mk & 0x10000u) && (R2.y < c.cutoff2);
+          const bool aA = (mrow & (1u << I)) && (R2.x < c.cutoff2);
+          const bool aB = (mrow & (0x10u << I)) && (R2.y < c.cutoff2);
           if (!__any_sync(0xffffffffu, aA || aB)) continue;
-          if (kLive) live |= ((aA ? 1u : 0u) | (aB ? 0x10000u : 0u)) << k;
-          const float2 TY = pA[256];
-          const int tyA = __float_as_int(TY.x), tyB = __float_as_int(TY.y);
-          const float2 abA = doBatch ? __ldg(&ljRow[ti + tyA]) : s_lj[ti + tyA];
-          const float2 abB = doBatch ? __ldg(&ljRow[ti + tyB]) : s_lj[ti + tyB];
-          const float2 QQ = mul2(f2(xi.w), pA[192]);
-          const float2 r2s = make_float2(aA ? R2.x : c.cutoff2, aB ? R2.y : c.cutoff2);
-          const float2 qqs = make_float2(aA ? QQ.x : 0.f, aB ? QQ.y : 0.f);
-          const float2 As = make_float2(aA ? abA.x : 0.f, aB ? abB.x : 0.f);
-          const float2 nBs = make_float2(aA ? -abA.y : 0.f, aB ? -abB.y : 0.f);
-          float2 F, FS;
-          pairForce2<doEnergy, doSlow>(r2s, qqs, As, nBs, c, F, FS, eV2);
-          // i: two partial sums; inactive elements add exact zeros
-          fix2 = fma2(DX, F, fix2);
-          fiy2 = fma2(DY, F, fiy2);
-          fiz2 = fma2(DZ, F, fiz2);
-          if (doSlow) {
-            fisx2 = fma2(DX, FS, fisx2);
-            fisy2 = fma2(DY, FS, fisy2);
-            fisz2 = fma2(DZ, FS, fisz2);
-          }
-          // j: bring P to step k and Q to step k+16 (one shift for both), subtract
-          const int src = (lane + (k - kLast)) & 31;
-          kLast = k;
-          PQx = make_float2(__shfl_sync(0xffffffffu, PQx.x, src), __shfl_sync(0xffffffffu, PQx.y, src));
-          PQy = make_float2(__shfl_sync(0xffffffffu, PQy.x, src), __shfl_sync(0xffffffffu, PQy.y, src));
-          PQz = make_float2(__shfl_sync(0xffffffffu, PQz.x, src), __shfl_sync(0xffffffffu, PQz.y, src));
-          PQx = fma2(neg2(DX), F, PQx);
-          PQy = fma2(neg2(DY), F, PQy);
-          PQz = fma2(neg2(DZ), F, PQz);
-          if (doSlow) {
-            PQsx = make_float2(__shfl_sync(0xffffffffu, PQsx.x, src),
-                               __shfl_sync(0xffffffffu, PQsx.y, src));
-            PQsy = make_float2(__shfl_sync(0xffffffffu, PQsy.x, src),
-                               __shfl_sync(0xffffffffu, PQsy.y, src));
-            PQsz = make_float2(__shfl_sync(0xffffffffu, PQsz.x, src),
-                               __shfl_sync(0xffffffffu, PQsz.y, src));
-            PQsx = fma2(neg2(DX), FS, PQsx);
-            PQsy = fma2(neg2(DY), FS, PQsy);
-            PQsz = fma2(neg2(DZ), FS, PQsz);
+          if (kLive) liveRow |= (aA ? 1u << I : 0u) | (aB ? 0x10u << I : 0u);
+          const int ti = __float_as_int(ib.w);
+          const int tA = ti + __float_as_int(tj.x), tB = ti + __float_as_int(tj.y);
+          const float2 abA = doBatch ? __ldg((const float2*)(ljRow + tA)) : ldShared2(adrLJ + tA);
+          const float2 abB = doBatch ? __ldg((const float2*)(ljRow + tB)) : ldShared2(adrLJ + tB);
+          const float2 QQ = make_float2(ib.z * jb.z, ib.z * jb.w);
+          float2 F, FS, E;
+          pairForce2<doEnergy, doSlow>(R2, QQ, make_float2(abA.x, abB.x),
+                                       make_float2(abA.y, abB.y), a.pk, F, FS, E);
+          // an element that is no interacting pair may hold anything, NaN
+          // included: it is replaced by an exact zero
+          F = make_float2(aA ? F.x : 0.f, aB ? F.y : 0.f);
+          if (doEnergy) eV2 = add2(eV2, make_float2(aA ? E.x : 0.f, aB ? E.y : 0.f));
+          fi[I][0] = fmaf(DX.y, F.y, fmaf(DX.x, F.x, fi[I][0]));
+          fi[I][1] = fmaf(DY.y, F.y, fmaf(DY.x, F.x, fi[I][1]));
+          fi[I][2] = fmaf(DZ.y, F.y, fmaf(DZ.x, F.x, fi[I][2]));
+          fj[0] = fma2(DX, F, fj[0]);
+          fj[1] = fma2(DY, F, fj[1]);
+          fj[2] = fma2(DZ, F, fj[2]);
+          if constexpr (doSlow) {
+            FS = make_float2(aA ? FS.x : 0.f, aB ? FS.y : 0.f);
+            fi[I][3] = fmaf(DX.y, FS.y, fmaf(DX.x, FS.x, fi[I][3]));
+            fi[I][4] = fmaf(DY.y, FS.y, fmaf(DY.x, FS.x, fi[I][4]));
+            fi[I][5] = fmaf(DZ.y, FS.y, fmaf(DZ.x, FS.x, fi[I][5]));
+            fj[3] = fma2(DX, FS, fj[3]);
+            fj[4] = fma2(DY, FS, fj[4]);
+            fj[5] = fma2(DZ, FS, fj[5]);
           }
         }
-        // rotate P (at step kLast) and Q (at step kLast+16) back to j = lane
-        float fjx, fjy, fjz, fjsx = 0.f, fjsy = 0.f, fjsz = 0.f;
-        {
-          const int srcP = (lane + 32 - kLast) & 31, srcQ = (lane + 16 - kLast) & 31;
-          fjx = __shfl_sync(0xffffffffu, PQx.x, srcP) + __shfl_sync(0xffffffffu, PQx.y, srcQ);
-          fjy = __shfl_sync(0xffffffffu, PQy.x, srcP) + __shfl_sync(0xffffffffu, PQy.y, srcQ);
-          fjz = __shfl_sync(0xffffffffu, PQz.x, srcP) + __shfl_sync(0xffffffffu, PQz.y, srcQ);
-          if (doSlow) {
-            fjsx = __shfl_sync(0xffffffffu, PQsx.x, srcP) + __shfl_sync(0xffffffffu, PQsx.y, srcQ);
-            fjsy = __shfl_sync(0xffffffffu, PQsy.x, srcP) + __shfl_sync(0xffffffffu, PQsy.y, srcQ);
-            fjsz = __shfl_sync(0xffffffffu, PQsz.x, srcP) + __shfl_sync(0xffffffffu, PQsz.y, srcQ);
+        if (kLive) live |= liveRow << J8;
+        // the row's j sums over the eight i lanes: lanes l and l ^ 4 hold the
+        // two j atoms in turned order, so each keeps its element x; then bit 1
+        // tells the fast from the slow force
+        float v[3], u[kNC];
+#pragma unroll
+        for (int q = 0; q < kNC; ++q) u[q] = fj[q].x + __shfl_xor_sync(0xffffffffu, fj[q].y, 4);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          if constexpr (doSlow) v[q] = keepHalf(u[q], u[q + 3], b1, 2);
+          else v[q] = u[q];
+        }
+        // the lane bits that are left tell rows apart: bit 0 the rows of a
+        // pair (with slow forces), else bit 1 the rows of a pair and bit 0
+        // the pairs. A last row without a partner is paired with zeros.
+        int Jrow = J8;
+        if (!(rows++ & 1)) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) held[q] = v[q];
+          Jheld = Jrow;
+          if (todo) continue;
+#pragma unroll
+          for (int q = 0; q < 3; ++q) v[q] = 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[q] = keepHalf(held[q], v[q], doSlow ? b0 : b1, doSlow ? 1 : 2);
+        Jrow = (doSlow ? b0 : b1) ? Jrow : Jheld;
+        if constexpr (!doSlow) {
+          if (rows <= 2) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) held2[q] = v[q];
+            Jheld2 = Jrow;
+            if (todo) continue;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v[q] = 0.f;
           }
+#pragma unroll
+          for (int q = 0; q < 3; ++q) v[q] = keepHalf(held2[q], v[q], b0, 1);
+          Jrow = b0 ? Jrow : Jheld2;
         }
-        const int jatom = jstart + lane;
-        if (fjx != 0.f || fjy != 0.f || fjz != 0.f) {
-          atomicAddFixed(&a.force[0 * (size_t)a.stride + jatom], toFixedForce(fjx));
-          atomicAddFixed(&a.force[1 * (size_t)a.stride + jatom], toFixedForce(fjy));
-          atomicAddFixed(&a.force[2 * (size_t)a.stride + jatom], toFixedForce(fjz));
+        // the lane's j atom, and its force array; F_j = -sum
+        if (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f) {
+          long long* f = a.force + (doSlow && b1 ? 3 * (size_t)a.stride : 0) + jstart + Jrow +
+                         (lane & 4) + lj;
+          atomicAddFixed(f, toFixedForce(-v[0]));
+          atomicAddFixed(f + (size_t)a.stride, toFixedForce(-v[1]));
+          atomicAddFixed(f + 2 * (size_t)a.stride, toFixedForce(-v[2]));
         }
-        if (doSlow && (fjsx != 0.f || fjsy != 0.f || fjsz != 0.f)) {
-          atomicAddFixed(&a.force[3 * (size_t)a.stride + jatom], toFixedForce(fjsx));
-          atomicAddFixed(&a.force[4 * (size_t)a.stride + jatom], toFixedForce(fjsy));
-          atomicAddFixed(&a.force[5 * (size_t)a.stride + jatom], toFixedForce(fjsz));
-        }
-        if (doEnergy) s_evg[wib][lane] += eV2.x + eV2.y;
       }
+      if (doEnergy) s_evg[wib][lane] += (eV2.x + eV2.y) * (-1.0f / 6.0f);  // the terms are -6 E
       if (kLive) a.liveOut[(size_t)jt * kWarp + lane] = live;
       if (((((jt - tl.jtileStart + 1) & (kFoldTiles - 1)) == 0) || jt == jtLast)) {
         // end of a tile group: its LJ energy and i forces into fixed point
@@ -579,15 +641,14 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
           s_ev[wib][lane] += toFixedEnergyF(s_evg[wib][lane]);
           s_evg[wib][lane] = 0.f;
         }
-        s_fi[wib][0][lane] += (long long)toFixedForce(fix2.x + fix2.y);
-        s_fi[wib][1][lane] += (long long)toFixedForce(fiy2.x + fiy2.y);
-        s_fi[wib][2][lane] += (long long)toFixedForce(fiz2.x + fiz2.y);
-        fix2 = fiy2 = fiz2 = f2(0.f);
-        if (doSlow) {
-          s_fi[wib][3][lane] += (long long)toFixedForce(fisx2.x + fisx2.y);
-          s_fi[wib][4][lane] += (long long)toFixedForce(fisy2.x + fisy2.y);
-          s_fi[wib][5][lane] += (long long)toFixedForce(fisz2.x + fisz2.y);
-          fisx2 = fisy2 = fisz2 = f2(0.f);
+        // i sums over the four j lanes: bits 4 and 3 keep cluster I = lane >> 3,
+        // so that every lane ends up with its own atom 8 I + li = lane
+#pragma unroll
+        for (int q = 0; q < kNC; ++q) {
+          const float lo = keepHalf(fi[0][q], fi[2][q], b4, 16);
+          const float hi = keepHalf(fi[1][q], fi[3][q], b4, 16);
+          s_fi[wib][q][lane] += (long long)toFixedForce(keepHalf(lo, hi, b3, 8));
+          fi[0][q] = fi[1][q] = fi[2][q] = fi[3][q] = 0.f;
         }
       }
       __syncwarp();

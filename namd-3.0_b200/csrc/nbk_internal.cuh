@@ -43,9 +43,6 @@ struct NbkConst {
   float beta;         // Ewald coefficient
   float beta2Pi;      // 2 beta / sqrt(pi)
   float one14;        // 1 - scale14
-  float pBeta;        // erfcShared's p times beta (packed steady-state math)
-  float gaussK;       // -beta^2 log2(e): exp(-beta^2 r^2) = 2^(gaussK r^2)
-  float s0;           // 0 with switching, 1 without (packed math: S = d^2 P + s0)
   int ljDim;          // LJ table row length
   int switching;      // 0 when switchdist >= cutoff (plain truncated LJ)
   double hAd, hBd;    // hA, hB in FP64 (precise kernel)
@@ -132,6 +129,23 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 
+// Shared-memory accesses by 32-bit address (a base held in a register and an
+// immediate offset), so that the pair loop forms no addresses.
+__device__ __forceinline__ unsigned sharedAddr(const void* p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ float4 ldShared4(const unsigned a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 ldShared2(const unsigned a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+
 // PTX approximate reciprocal, base-2 exponential and reciprocal square root
 // (rcp/ex2/rsqrt.approx.ftz.f32). The inputs here are normal numbers (r^2 is
 // at least the square of the shortest pair distance, 2^(gaussK r^2) lies in
@@ -160,6 +174,19 @@ __device__ __forceinline__ double rsqrtApprox64(double x) {
   return y;
 }
 
+// Constants of the packed pair math (makePacked, nbk_consts.cu); those that a
+// packed instruction reads are held twice. With d = min(rc^2 - r^2, D), D =
+// rc^2 - rs^2 and c1 = 1/D^3 the switch is S = c1 d^2 (3 D - 2 d) and (dS/dr)/r
+// = 12 c1 d (d - D) = T, so -6 S = d (T - 6 c1 D d). Without switching d = D =
+// 1 for every pair, which gives S = 1 and T = 0 exactly.
+struct PackedConst {
+  float2 dA, dB, hA;    // -12 c1 D, 12 c1, -6 c1 D
+  float2 rc3inv;
+  float2 nBeta2Pi;      // -2 beta / sqrt(pi)
+  float rc2, dMax;      // rc^2 (huge without switching), D
+  float pBeta, gaussK;  // erfcShared's p times beta; exp(-beta^2 r^2) = 2^(gaussK r^2)
+};
+
 // FP32 pair math for two pairs (x and y elements); nB = -B. F, FS = (dE/dr)/r
 // of LJ + fast electrostatics and of the slow (PME real-space remainder)
 // electrostatics; the caller applies F_i += F (x_j - x_i), F_j -= F (x_j - x_i).
@@ -167,49 +194,47 @@ __device__ __forceinline__ double rsqrtApprox64(double x) {
 //   fast    E = qq (1/r - (3 - r^2/rc^2)/(2 rc))
 //   slow    E = qq ((3 - r^2/rc^2)/(2 rc) + (erfc(beta r) - 1)/r)
 // (src/CudaComputeNonbondedInteractions.h:37-159 states the same forms.) Only
-// the LJ energy is summed here (doVdwEnergy): the electrostatic energies and
-// the slow virial are formed in FP64 by the precise kernel (nbk_force.cu).
-// An element with qq = A = nB = 0 and r2 = cutoff^2 contributes exactly zero
-// to F, FS and the energy, which is how callers switch a pair off without a
-// branch. The slow term regroups the same quantities: with x = beta r,
-// t = 1/(1 + p x) and e = exp(-x^2) = 2^(gaussK r^2), erfc = t P(t) e and the
-// force factor erfc + (2 beta/sqrt(pi)) r e = (t P(t) + (2 beta/sqrt(pi)) r) e.
+// the LJ energy is formed here (doVdwEnergy; e6 = -6 E): the electrostatic
+// energies and the slow virial are formed in FP64 by the precise kernel
+// (nbk_force.cu). Callers replace the results of an element that is no
+// interacting pair. LJ is taken as r^-6 [(2 A r^-6 - B) (-6 S/r^2) + (A r^-6 -
+// B) (dS/dr)/r], which needs the fewest operations. The slow term regroups the
+// same quantities: with x = beta r, t = 1/(1 + p x) and e = exp(-x^2) =
+// 2^(gaussK r^2), erfc = t P(t) e and the force factor erfc + (2
+// beta/sqrt(pi)) r e = (t P(t) + (2 beta/sqrt(pi)) r) e; the bracket is formed
+// with its sign turned.
 template <bool doVdwEnergy, bool doSlow>
 __device__ __forceinline__ void pairForce2(const float2 r2, const float2 qq, const float2 A,
-                                           const float2 nB, const NbkConst& c, float2& f,
-                                           float2& fs, float2& eVdw) {
+                                           const float2 nB, const PackedConst& c, float2& f,
+                                           float2& fs, float2& e6) {
   const float2 rinv = make_float2(rsqrtApprox(r2.x), rsqrtApprox(r2.y));
   const float2 rinv2 = mul2(rinv, rinv);
-  const float2 rinv6 = mul2(mul2(rinv2, rinv2), rinv2);
   const float2 rinv3 = mul2(rinv, rinv2);
-  const float2 ab6 = fma2(A, rinv6, nB);
-  const float2 w = mul2(ab6, rinv6);
-  const float2 dw = mul2(fma2(A, rinv6, ab6), mul2(mul2(f2(-6.0f), rinv2), rinv6));
-  // switch without a branch: without switching rs2 = rc2 and lj0..lj3 = 0,
-  // so d = 0 for every pair inside the cutoff and S = s0 = 1, dS = 0
-  const float2 t2 = make_float2(fmaxf(r2.x, c.rs2), fmaxf(r2.y, c.rs2));
-  const float2 d = add2(f2(c.rc2), neg2(t2));
-  const float2 s = fma2(mul2(d, d), fma2(f2(c.lj1), t2, f2(c.lj0)), f2(c.s0));
-  const float2 ds = mul2(d, fma2(f2(c.lj2), t2, f2(c.lj3)));
-  f = fma2(w, ds, mul2(dw, s));
-  f = fma2(qq, add2(f2(c.rc3inv), neg2(rinv3)), f);
-  if (doVdwEnergy) eVdw = fma2(w, s, eVdw);
+  const float2 rinv6 = mul2(rinv3, rinv3);
+  // scalar: A and B of the two pairs come from two table entries
+  const float2 ab6 = make_float2(fmaf(A.x, rinv6.x, nB.x), fmaf(A.y, rinv6.y, nB.y));
+  const float2 ab12 = make_float2(fmaf(A.x, rinv6.x, ab6.x), fmaf(A.y, rinv6.y, ab6.y));
+  const float2 d = make_float2(fminf(c.rc2 - r2.x, c.dMax), fminf(c.rc2 - r2.y, c.dMax));
+  const float2 ds = mul2(d, fma2(c.dB, d, c.dA));
+  const float2 s6 = mul2(d, fma2(c.hA, d, ds));
+  const float2 lj = fma2(ab12, mul2(rinv2, s6), mul2(ab6, ds));
+  f = fma2(lj, rinv6, mul2(qq, add2(c.rc3inv, neg2(rinv3))));
+  if (doVdwEnergy) e6 = mul2(mul2(ab6, rinv6), s6);
   if (doSlow) {
     const float2 r = mul2(r2, rinv);
-    const float2 den = fma2(f2(c.pBeta), r, f2(1.0f));
-    const float2 t = make_float2(rcpApprox(den.x), rcpApprox(den.y));
-    const float2 g = mul2(r2, f2(c.gaussK));
-    const float2 ex = make_float2(ex2Approx(g.x), ex2Approx(g.y));
-    float2 q = f2(kErfcC0);
-    q = fma2(q, t, f2(kErfcC1));
-    q = fma2(q, t, f2(kErfcC2));
-    q = fma2(q, t, f2(kErfcC3));
-    q = fma2(q, t, f2(kErfcC4));
-    q = fma2(q, t, f2(kErfcC5));
-    q = fma2(q, t, f2(kErfcC6));
-    q = fma2(q, t, f2(kErfcC7));
-    const float2 corr = mul2(fma2(f2(c.beta2Pi), r, mul2(t, q)), ex);
-    fs = mul2(qq, fma2(add2(f2(1.0f), neg2(corr)), rinv3, f2(-c.rc3inv)));
+    const float2 t = make_float2(rcpApprox(fmaf(c.pBeta, r.x, 1.0f)),
+                                 rcpApprox(fmaf(c.pBeta, r.y, 1.0f)));
+    const float2 ex = make_float2(ex2Approx(r2.x * c.gaussK), ex2Approx(r2.y * c.gaussK));
+    float2 q = f2(-kErfcC0);
+    q = fma2(q, t, f2(-kErfcC1));
+    q = fma2(q, t, f2(-kErfcC2));
+    q = fma2(q, t, f2(-kErfcC3));
+    q = fma2(q, t, f2(-kErfcC4));
+    q = fma2(q, t, f2(-kErfcC5));
+    q = fma2(q, t, f2(-kErfcC6));
+    q = fma2(q, t, f2(-kErfcC7));
+    const float2 nCorr = fma2(c.nBeta2Pi, r, mul2(t, q));
+    fs = mul2(qq, fma2(fma2(nCorr, ex, f2(1.0f)), rinv3, neg2(c.rc3inv)));
   } else {
     fs = f2(0.0f);
   }
@@ -234,6 +259,19 @@ constexpr int kSlowTableDeg = 5;
 constexpr int kSlowTableDeg1 = kSlowTableDeg + 1;  // coefficients per row
 constexpr int kSlowTableRow = 6;  // doubles per row of the global copy
 constexpr double kSlowTableTol = 1e-12;  // fit error, relative to max |phi_s| + 1/rc
+
+// Puts the 32 x 32 bits of a tile held as rows (lane i: bit j) into block order
+// (lane l: bit 8 J + 4 e + I <-> i = 8 I + (l & 7), j = 8 J + (4 e ^ (l & 4)) +
+// (l >> 3), the force kernel's order), or back: the two orders exchange I and
+// l >> 3 and swap neighbouring nibbles of lanes with bit 2 set, so the same
+// exchange is its own inverse. All lanes call.
+__device__ __forceinline__ unsigned blockOrder(const unsigned w, const int lane) {
+  unsigned out = 0;
+#pragma unroll
+  for (int I = 0; I < 4; ++I)
+    out |= ((__shfl_sync(0xffffffffu, w, 8 * I + (lane & 7)) >> (lane >> 3)) & 0x11111111u) << I;
+  return (lane & 4) ? ((out >> 4) & 0x0f0f0f0fu) | ((out & 0x0f0f0f0fu) << 4) : out;
+}
 
 // Component k (0..8, row-major 3x3) of a symmetric tensor stored as
 // xx, xy, xz, yy, yz, zz.
@@ -279,7 +317,7 @@ struct ForceArgs {
   const int* numListsDev;      // device count (compacted lists) or NULL
   int numListsHost;            // used when numListsDev == NULL
   const int* tileJatomStart;
-  nbk_tile_excl* tileExcls;    // read by the force kernel, written by refineKernel
+  nbk_tile_excl* tileExcls;    // block order; read by the force kernel, written by refineKernel
   int* jtileActive;            // refineKernel: written
   int* listActive;             // refineKernel: number of active j-tiles per list
   const PatchPair* patchPairs; // refineKernel
@@ -292,6 +330,7 @@ struct ForceArgs {
   const float2* ljTable;       // [ljDim*ljDim] (A, B) * scaling
   float3 lata, latb, latc;
   NbkConst c;
+  PackedConst pk;              // force kernel
   long long* force;            // SoA [6][stride] fixed point
   int stride;
   long long* acc;              // [kAccCount]
@@ -302,11 +341,11 @@ struct ForceArgs {
   int slowTableRows;
   double slowStep, slowInvStep;  // table step D (a power of two) and 1/D
   unsigned* liveOut;           // [numJtiles][32] interacting-pair words (force kernel writes,
-                               // precise kernel reads)
+                               // precise kernel reads), block order
   // replicas (batched evaluation; all NULL for a single system)
   const int* compRep;          // [numComputes] replica of each compute
   const float3* repLat;        // [3*numReplicas] lattice vectors a, b, c
-  const float2* repLJ;         // [numReplicas][ljDim*ljDim] (A, B) * scaling
+  const float2* repLJ;         // [numReplicas][ljDim*ljDim] (A, -B) * scaling
 };
 
 }  // namespace nbk

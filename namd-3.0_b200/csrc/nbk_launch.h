@@ -13,6 +13,7 @@ namespace nbk {
 // Pair-math constants from the caller's parameters (nbk_consts.cu); shared by
 // the handle and by the allocation-free entry point.
 void makeConstants(const nbk_params& p, int ljDim, NbkConst& c, NbkConst64& k);
+void makePacked(const NbkConst64& k, PackedConst& c);
 // The FP64 slow-term table of the force kernel's precise pass; returns rows.
 int buildSlowTable(double beta, double cutoff, double pairlistdist, std::vector<double>& out,
                    double* step);

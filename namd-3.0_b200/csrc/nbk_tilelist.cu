@@ -186,8 +186,8 @@ __global__ void __launch_bounds__(kCompactWarps * 32)
 }
 
 // Pairlist refinement without force math: for every j tile of every culled
-// list, bit t of TileExcl.excl[lane] is set when the pair (i = iatomStart +
-// lane, j = jatomStart + ((lane + t) & 31)) lies within the pairlist cutoff
+// list, the bit of a pair (i, j) of the tile, in block order (blockOrder), is
+// set when the pair lies within the pairlist cutoff
 // (FP32 r^2 with the shift and operand order of shiftOf / dist2), is not a
 // padding pair, is not the diagonal or lower triangle of a self tile and is
 // not a full exclusion (the pairlist pass of nonbondedForceKernel,
@@ -201,9 +201,8 @@ __global__ void __launch_bounds__(kCompactWarps * 32)
 // tile's coordinates and indices read as warp-wide broadcasts from shared
 // memory. The sign bits of r^2 - plcutoff^2 (the same per-element rounding
 // as dist2; the sign of a rounded difference is the sign of the exact one)
-// are shifted into a word whose bit j marks pair (lane, j); one rotation by
-// the lane number turns it into the TileExcl order (bit t <-> j = (lane + t)
-// & 31). Exclusions are only looked up for candidates whose global indices
+// are shifted into a word whose bit j marks pair (lane, j); four shuffles put
+// the tile's words into block order. Exclusions are only looked up for candidates whose global indices
 // lie within the i atom's maxdiff window: |jIndex - iIndex| <= maxdiff is
 // tested as the sign of (jIndex - iIndex)^2 - (maxdiff^2 + 1/2) in FP32,
 // exact while indices are below 2^24 and maxdiff <= kFpWindowMaxDiff (the
@@ -323,9 +322,8 @@ __global__ void __launch_bounds__(128) refineKernel(const __grid_constant__ Forc
             }
           }
         }
-        const unsigned m = __funnelshift_r(mw, mw, lane);  // bit t <-> j = (lane + t) & 31
-        a.tileExcls[jt].excl[lane] = m;
-        const bool any = __any_sync(0xffffffffu, m != 0);
+        a.tileExcls[jt].excl[lane] = blockOrder(mw, lane);
+        const bool any = __any_sync(0xffffffffu, mw != 0);
         if (lane == 0) a.jtileActive[jt] = any ? 1 : 0;
         activeTiles += any ? 1 : 0;
         __syncwarp();
