@@ -120,11 +120,10 @@ struct nbk_context {
   DBuf<nbk_tile_list> lists1;
   DBuf<PatchPair> patchPairs;
   DBuf<int> jatom1;
-  DBuf<nbk_tile_excl> excl1;
-  DBuf<int> jtileActive, listActive;
+  DBuf<int> listActive;
   // compacted lists for steady-state evaluations
-  DBuf<nbk_tile_list> lists2;      // refined, compacted lists, longest first
-  DBuf<nbk_tile_list> listsCompact;  // the compaction's output before the sort
+  DBuf<nbk_tile_list> lists2;      // refined lists that kept tiles, longest first
+  DBuf<nbk_tile_list> listsCompact;  // the same in their own order (batched replicas)
   // Batched replicas skip the sort: lists in compaction order stay grouped by
   // replica (per-replica LJ rows and accumulators stay hot), and a launch
   // over many replicas holds enough lists that its tail is short anyway.
@@ -414,8 +413,6 @@ NBK_API int nbk_destroy(nbk_handle h) {
   h->lists1.release();
   h->patchPairs.release();
   h->jatom1.release();
-  h->excl1.release();
-  h->jtileActive.release();
   h->listActive.release();
   h->lists2.release();
   h->listsCompact.release();
@@ -615,8 +612,6 @@ NBK_API int nbk_build_tile_lists(nbk_handle h, int numPatches, int atomStorageSi
   NBK_CUDA(h->patchPairs.ensure(nl), "nbk_build_tile_lists");
   NBK_CUDA(h->listActive.ensure(nl), "nbk_build_tile_lists");
   NBK_CUDA(h->jatom1.ensure(nj), "nbk_build_tile_lists");
-  NBK_CUDA(h->excl1.ensure(nj), "nbk_build_tile_lists");
-  NBK_CUDA(h->jtileActive.ensure(nj), "nbk_build_tile_lists");
   NBK_CUDA(launchBBoxes(atomStorageSize / 32, h->xyzq, h->bboxes.p, st), "bounding boxes");
   h->launches += 2;
   // culling distance: the pairlist cutoff inflated by a relative 1e-5 so FP32
@@ -679,35 +674,41 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
   a.splitLog2 = h->tuneSplitLog2[key];
   NBK_CUDA(timedEvent(h, kTimedStart, st), "timing event");
   if (pairlist) {
-    // refinement of the culled lists (the pairlist pass), then their
-    // compaction (reSortTileLists), both on the device
+    // refinement of the culled lists (the pairlist pass) and the order of
+    // those that keep tiles (reSortTileLists), both on the device
+    const int nl = std::max(h->numLists, 1), nj = std::max(h->jcap, 1);
+    h->listsSorted = h->nrep == 0;
+    if (h->listsSorted) {
+      NBK_CUDA(h->lists2.ensure(nl), "nbk_nonbonded_force");
+      NBK_CUDA(h->lenHist.ensure((size_t)h->maxListLen + 1), "nbk_nonbonded_force");
+      NBK_CUDA(cudaMemsetAsync(h->lenHist.p, 0, sizeof(int) * ((size_t)h->maxListLen + 1), st),
+               "nbk_nonbonded_force");
+    } else {
+      NBK_CUDA(h->listsCompact.ensure(nl), "nbk_nonbonded_force");
+    }
+    NBK_CUDA(h->jatom2.ensure(nj), "nbk_nonbonded_force");
+    NBK_CUDA(h->excl2.ensure(nj), "nbk_nonbonded_force");
     ForceArgs r = a;
     r.lists = h->lists1.p;
     r.numListsDev = nullptr;
     r.numListsHost = h->numLists;
     r.tileJatomStart = h->jatom1.p;
-    r.tileExcls = h->excl1.p;
-    r.jtileActive = h->jtileActive.p;
+    r.tileJatomOut = h->jatom2.p;
+    r.tileExcls = h->excl2.p;
     r.listActive = h->listActive.p;
     r.patchPairs = h->patchPairs.p;
     r.workCounter = h->counters.p + 3;
-    NBK_CUDA(cudaMemsetAsync(h->counters.p + 3, 0, sizeof(int), st), "nbk_nonbonded_force");
+    // lists and tiles kept; with them the work counters of all three kernels
+    NBK_CUDA(cudaMemsetAsync(h->counters.p, 0, sizeof(int) * 5, st), "nbk_nonbonded_force");
     NBK_CUDA(launchRefine(r, h->numSM, st), "pairlist refinement");
-    const int nl = std::max(h->numLists, 1), nj = std::max(h->jcap, 1);
-    NBK_CUDA(h->lists2.ensure(nl), "nbk_nonbonded_force");
-    NBK_CUDA(h->listsCompact.ensure(nl), "nbk_nonbonded_force");
-    NBK_CUDA(h->lenHist.ensure((size_t)h->maxListLen + 1), "nbk_nonbonded_force");
-    NBK_CUDA(h->jatom2.ensure(nj), "nbk_nonbonded_force");
-    NBK_CUDA(h->excl2.ensure(nj), "nbk_nonbonded_force");
-    NBK_CUDA(cudaMemsetAsync(h->counters.p, 0, sizeof(int) * 2, st), "nbk_nonbonded_force");
-    NBK_CUDA(launchCompact(h->numLists, h->lists1.p, h->listActive.p, h->jtileActive.p, h->jatom1.p,
-                           h->excl1.p, h->listsCompact.p, h->jatom2.p, h->excl2.p, h->counters.p,
-                           h->numSM, st), "tile-list compaction");
-    h->listsSorted = h->nrep == 0;
     if (h->listsSorted) {
-      NBK_CUDA(launchSortLists(h->numLists, h->listsCompact.p, h->counters.p, h->maxListLen,
-                               h->lenHist.p, h->lists2.p, h->numSM, st), "tile-list sort");
-      h->launches += 3;
+      NBK_CUDA(launchSortLists(h->numLists, h->lists1.p, h->listActive.p, h->maxListLen,
+                               h->lenHist.p, h->counters.p, h->lists2.p, h->numSM, st),
+               "tile-list sort");
+      h->launches += 1;
+    } else {
+      NBK_CUDA(launchCompact(h->numLists, h->lists1.p, h->listActive.p, h->listsCompact.p,
+                             h->counters.p, h->numSM, st), "tile-list compaction");
     }
     h->launches += 2;
     h->refined = true;
@@ -716,12 +717,16 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
   a.lists = h->refinedLists();
   a.tileJatomStart = h->jatom2.p;
   a.tileExcls = h->excl2.p;
-  NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int) * 3, st), "nbk_nonbonded_force");
+  if (!pairlist)
+    NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int) * 3, st), "nbk_nonbonded_force");
   if (needsPrecise(flags)) {
     NBK_CUDA(h->live.ensure((size_t)std::max(h->jcap, 1) * 32), "nbk_nonbonded_force");
     a.liveOut = h->live.p;
   }
   NBK_CUDA(launchForce(a, flags, h->tuneMinBlocks[key], h->numSM, st), "force kernel");
+    r.lenHist = h->listsSorted ? h->lenHist.p : nullptr;
+    r.maxLen = h->maxListLen;
+    r.counts = h->counters.p;
   h->launches += 1;
   NBK_CUDA(timedEvent(h, kTimedMid, st), "timing event");
   const bool corrections = (flags & NBK_CORRECTIONS) && (h->numMod || h->numExc);
@@ -863,25 +868,36 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
   NBK_CUDA(cudaStreamSynchronize(st), "export");
   *numTileLists = cnt[0];
   *numJtiles = cnt[1];
-  if (tl && cnt[0])
-    NBK_CUDA(cudaMemcpy(tl, h->refinedLists(), sizeof(nbk_tile_list) * cnt[0], cudaMemcpyDeviceToHost), "export");
-  if (jatom && cnt[1])
-    NBK_CUDA(cudaMemcpy(jatom, h->jatom2.p, sizeof(int) * cnt[1], cudaMemcpyDeviceToHost), "export");
-  if (excl && cnt[1])
-  {
-    NBK_CUDA(cudaMemcpy(excl, h->excl2.p, sizeof(nbk_tile_excl) * cnt[1], cudaMemcpyDeviceToHost), "export");
-    // from block order to the interface's: bit t of lane i <-> j = (i + t) & 31
-    for (int k = 0; k < cnt[1]; ++k) {
-      unsigned w[32];
-      std::memcpy(w, excl[k].excl, sizeof(w));
-      for (int i = 0; i < 32; ++i) {
-        unsigned row = 0;
-        for (int lj = 0; lj < 4; ++lj)
-          row |= ((w[8 * lj + (i & 7)] >> (i >> 3)) & 0x11111111u) << lj;
-        if (i & 4) row = ((row >> 4) & 0x0f0f0f0fu) | ((row & 0x0f0f0f0fu) << 4);
-        excl[k].excl[i] = (row >> i) | (i ? row << (32 - i) : 0u);
-      }
-    }
+  if (!cnt[0] || (!tl && !jatom && !excl)) return NBK_OK;
+  // a list's tiles lie in slots of its own; the export closes the gaps
+  std::vector<nbk_tile_list> lists(cnt[0]);
+  NBK_CUDA(cudaMemcpy(lists.data(), h->refinedLists(), sizeof(nbk_tile_list) * cnt[0],
+                      cudaMemcpyDeviceToHost), "export");
+  std::vector<int> to(cnt[0]);
+  int next = 0;
+  for (int k = 0; k < cnt[0]; ++k) {
+    to[k] = next;
+    next += lists[k].jtileEnd - lists[k].jtileStart + 1;
+  }
+  if (jatom || excl) {
+    DBuf<int> dTo, dJatom;
+    DBuf<nbk_tile_excl> dExcl;
+    cudaError_t e = dTo.ensure(cnt[0]);
+    if (e == cudaSuccess) e = dJatom.ensure(std::max(next, 1));
+    if (e == cudaSuccess) e = dExcl.ensure(std::max(next, 1));
+    if (e == cudaSuccess) e = cudaMemcpy(dTo.p, to.data(), sizeof(int) * cnt[0], cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+      e = launchExportTiles(cnt[0], h->refinedLists(), dTo.p, h->jatom2.p, h->excl2.p, dJatom.p,
+                            dExcl.p, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && jatom)
+      e = cudaMemcpy(jatom, dJatom.p, sizeof(int) * next, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && excl)
+      e = cudaMemcpy(excl, dExcl.p, sizeof(nbk_tile_excl) * next, cudaMemcpyDeviceToHost);
+    dTo.release();
+    dJatom.release();
+    dExcl.release();
+    NBK_CUDA(e, "export");
   }
   return NBK_OK;
 }
@@ -916,6 +932,13 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
   NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int), st), "nbk_adjoint");
   AdjArgs a{};
   a.lists = h->refinedLists();
+  if (tl)
+    for (int k = 0; k < cnt[0]; ++k) {
+      const int n = lists[k].jtileEnd - lists[k].jtileStart + 1;
+      lists[k].jtileStart = to[k];
+      lists[k].jtileEnd = to[k] + n - 1;
+      tl[k] = lists[k];
+    }
   a.numListsDev = h->counters.p;
   a.tileJatomStart = h->jatom2.p;
   a.tileExcls = h->excl2.p;

@@ -318,8 +318,11 @@ struct ForceArgs {
   int numListsHost;            // used when numListsDev == NULL
   const int* tileJatomStart;
   nbk_tile_excl* tileExcls;    // block order; read by the force kernel, written by refineKernel
-  int* jtileActive;            // refineKernel: written
-  int* listActive;             // refineKernel: number of active j-tiles per list
+  int* tileJatomOut;           // refineKernel: j-tile starts of the tiles it keeps
+  int* listActive;             // refineKernel: number of tiles kept per list
+  int* lenHist;                // refineKernel: lists by length 1..maxLen (clamped), or NULL
+  int maxLen;
+  int* counts;                 // refineKernel: counts[1] += tiles kept
   const PatchPair* patchPairs; // refineKernel
   const float4* xyzq;
   const int* vdwTypes;

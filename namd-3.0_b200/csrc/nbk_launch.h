@@ -14,6 +14,8 @@ namespace nbk {
 // the handle and by the allocation-free entry point.
 void makeConstants(const nbk_params& p, int ljDim, NbkConst& c, NbkConst64& k);
 void makePacked(const NbkConst64& k, PackedConst& c);
+int buildForceTable(double beta, double cutoff, double pairlistdist, std::vector<float4>& out,
+                    double* step);
 // The FP64 slow-term table of the force kernel's precise pass; returns rows.
 int buildSlowTable(double beta, double cutoff, double pairlistdist, std::vector<double>& out,
                    double* step);
@@ -27,13 +29,16 @@ cudaError_t launchForce(const ForceArgs& a, unsigned flags, int minBlocks, int n
 bool needsPrecise(unsigned flags);
 cudaError_t launchPrecise(const ForceArgs& a, unsigned flags, int numSM, cudaStream_t st);
 // Pairlist refinement of the culled lists a.lists[0, a.numListsHost): writes
-// a.tileExcls, a.jtileActive, a.listActive and the excluded-pair counts.
+// a.tileExcls, a.tileJatomOut, a.listActive, a.lenHist (unless NULL),
+// a.counts[1] (tiles kept) and the excluded-pair counts.
 cudaError_t launchRefine(const ForceArgs& a, int numSM, cudaStream_t st);
 
-// The compacted lists [0, *numListsDev) of src copied to dst in order of
-// decreasing j-tile count (lengths clamped to maxLen); hist: maxLen + 1 ints.
-cudaError_t launchSortLists(int numListsMax, const nbk_tile_list* src, const int* numListsDev,
-                            int maxLen, int* hist, nbk_tile_list* dst, int numSM, cudaStream_t st);
+// The lists of src that kept tiles (listActive), as dst in order of decreasing
+// j-tile count; hist: their counts by length 1..maxLen (clamped), used up as
+// cursors; counts[0] receives their number.
+cudaError_t launchSortLists(int numLists, const nbk_tile_list* src, const int* listActive,
+                            int maxLen, int* hist, int* counts, nbk_tile_list* dst, int numSM,
+                            cudaStream_t st);
 
 cudaError_t launchBBoxes(int numTiles, const float4* xyzq, BBox* bb, cudaStream_t st);
 
@@ -44,10 +49,15 @@ cudaError_t launchBuildLists(int numLists, const ListSeed* seeds,
                              nbk_tile_list* lists, PatchPair* pp, int* tileJatomStart,
                              cudaStream_t st);
 
+// The same lists in their own order (counters[0] zeroed before).
 cudaError_t launchCompact(int numLists, const nbk_tile_list* src, const int* listActive,
-                          const int* jtileActive, const int* jatomSrc, const nbk_tile_excl* exclSrc,
-                          nbk_tile_list* dst, int* jatomDst, nbk_tile_excl* exclDst, int* counters,
-                          int numSM, cudaStream_t st);
+                          nbk_tile_list* dst, int* counters, int numSM, cudaStream_t st);
+
+// Tiles of the refined lists into packed arrays (list k's at dst[k]) in the
+// interface's bit order.
+cudaError_t launchExportTiles(int numLists, const nbk_tile_list* lists, const int* dst,
+                              const int* jatom, const nbk_tile_excl* excl, int* jatomOut,
+                              nbk_tile_excl* exclOut, cudaStream_t st);
 
 struct CorrArgs {
   const nbk_exclusion* modified;
@@ -111,6 +121,10 @@ struct AdjArgs {
   float cV, cE, cS;
   float3 lata, latb, latc;
   NbkConst c;
+  PackedConst pk;
+  const float4* slowTable;  // phi_s rows rounded to FP32: (c0..c3), (c4, c5, -, -)
+  int slowRows, tabCopies;  // tabCopies: set by the launch
+  float slowStep, slowInvStep;
   long long* grad;       // SoA [4][stride]: gx, gy, gz, gq (fixed point, force scale)
   int stride;
   double* gradAB;        // [2][ljDim*ljDim] (FP64 atomics)

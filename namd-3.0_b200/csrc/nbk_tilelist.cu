@@ -117,71 +117,40 @@ __global__ void buildListsKernel(int numLists, const ListSeed* __restrict__ seed
   }
 }
 
-// After the pairlist refinement: drop j tiles without interacting pairs and
-// lists left empty (reSortTileLists' compaction, src/CudaTileListKernel.cu:
-// 1605-1665). counters[0] = lists kept, counters[1] = j tiles kept. A block
-// of kCompactWarps warps takes as many lists at a time, one per warp; one
-// thread reserves the output of all of them with one pair of atomics.
-constexpr int kCompactWarps = 8;
+// After the pairlist refinement: the lists that kept tiles, in their order
+// (batched replicas, whose lists stay grouped by replica). A block of
+// kCompactWarps warps takes as many lists at a time as it has threads; one
+// thread reserves the output of all of them with one atomic on counters[0].
+constexpr int kCompactThreads = 256;
 
-__global__ void __launch_bounds__(kCompactWarps * 32)
+__global__ void __launch_bounds__(kCompactThreads)
     compactKernel(int numLists, const nbk_tile_list* __restrict__ src,
-                  const int* __restrict__ listActive, const int* __restrict__ jtileActive,
-                  const int* __restrict__ jatomSrc, const nbk_tile_excl* __restrict__ exclSrc,
-                  nbk_tile_list* __restrict__ dst, int* __restrict__ jatomDst,
-                  nbk_tile_excl* __restrict__ exclDst, int* __restrict__ counters) {
-  __shared__ int s_n[kCompactWarps], s_pos[kCompactWarps], s_jpos[kCompactWarps];
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  for (int Lb = blockIdx.x * kCompactWarps; Lb < numLists; Lb += gridDim.x * kCompactWarps) {
-    const int L = Lb + wib;
-    int n = 0;
-    nbk_tile_list s;
-    if (L < numLists) {
-      s = src[L];
-      // listActive is only written for lists with tiles (empty lists skip the refinement)
-      if (s.jtileEnd >= s.jtileStart) n = listActive[L];
-    }
-    if (lane == 0) s_n[wib] = n;
+                  const int* __restrict__ listActive, nbk_tile_list* __restrict__ dst,
+                  int* __restrict__ counters) {
+  __shared__ int s_n[kCompactThreads / 32], s_base;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  for (int L0 = blockIdx.x * kCompactThreads; L0 < numLists; L0 += gridDim.x * kCompactThreads) {
+    const int L = L0 + threadIdx.x;
+    const int len = L < numLists ? listActive[L] : 0;
+    const unsigned ball = __ballot_sync(0xffffffffu, len > 0);
+    if (lane == 0) s_n[wib] = __popc(ball);
     __syncthreads();
     if (threadIdx.x == 0) {
-      int kept = 0, tiles = 0;
-      for (int w = 0; w < kCompactWarps; ++w) {
-        s_pos[w] = kept;
-        s_jpos[w] = tiles;
-        kept += s_n[w] > 0 ? 1 : 0;
-        tiles += s_n[w];
+      int kept = 0;
+      for (int w = 0; w < kCompactThreads / 32; ++w) {
+        const int n = s_n[w];
+        s_n[w] = kept;
+        kept += n;
       }
-      const int p0 = kept ? atomicAdd(&counters[0], kept) : 0;
-      const int j0 = kept ? atomicAdd(&counters[1], tiles) : 0;
-      for (int w = 0; w < kCompactWarps; ++w) {
-        s_pos[w] += p0;
-        s_jpos[w] += j0;
-      }
+      s_base = kept ? atomicAdd(&counters[0], kept) : 0;
     }
     __syncthreads();
-    if (n > 0) {  // warp-uniform
-      const int pos = s_pos[wib], jpos = s_jpos[wib];
-      int w = 0;
-      for (int j0 = s.jtileStart; j0 <= s.jtileEnd; j0 += 32) {
-        const int jt = j0 + lane;
-        const bool act = (jt <= s.jtileEnd) && jtileActive[jt];
-        unsigned ball = __ballot_sync(0xffffffffu, act);
-        if (act) jatomDst[jpos + w + __popc(ball & ((1u << lane) - 1u))] = jatomSrc[jt];
-        while (ball) {
-          const int b = __ffs(ball) - 1;
-          ball &= ball - 1;
-          exclDst[jpos + w].excl[lane] = exclSrc[j0 + b].excl[lane];
-          ++w;
-        }
-      }
-      if (lane == 0) {
-        nbk_tile_list d = s;
-        d.jtileStart = jpos;
-        d.jtileEnd = jpos + n - 1;
-        dst[pos] = d;
-      }
+    if (len > 0) {
+      nbk_tile_list t = src[L];
+      t.jtileEnd = t.jtileStart + len - 1;
+      dst[s_base + s_n[wib] + __popc(ball & ((1u << lane) - 1u))] = t;
     }
+    __syncthreads();
   }
 }
 
@@ -191,10 +160,14 @@ __global__ void __launch_bounds__(kCompactWarps * 32)
 // (FP32 r^2 with the shift and operand order of shiftOf / dist2), is not a
 // padding pair, is not the diagonal or lower triangle of a self tile and is
 // not a full exclusion (the pairlist pass of nonbondedForceKernel,
-// src/CudaComputeNonbondedKernel.cu:1202-1249,1424-1443). Writes the masks
-// in place, jtileActive / listActive for the compaction and the per-replica
-// count of excluded pairs within the pairlist cutoff. One warp per list,
-// lists handed out from a.workCounter.
+// src/CudaComputeNonbondedKernel.cu:1202-1249,1424-1443). The tiles that keep
+// pairs are written, closed up, to the start of the list's own slots of
+// a.tileExcls / a.tileJatomOut (the compaction of reSortTileLists,
+// src/CudaTileListKernel.cu:1605-1665, without a pass that moves the 128-byte
+// masks once more: 36 us at 92,224 atoms); their number goes to listActive and
+// the histogram of lengths, and the excluded pairs within the pairlist cutoff
+// are counted per replica. One warp per list, lists handed out from
+// a.workCounter.
 //
 // Layout of the work: every lane tests its i atom against j = 0..31 in
 // natural order, two j atoms (k, k + 16) per packed-FP32 step, with the j
@@ -220,14 +193,17 @@ __global__ void __launch_bounds__(128) refineKernel(const __grid_constant__ Forc
   const float2 nPlc2 = f2(-a.c.plcutoff2);
   float* const p0 = reinterpret_cast<float*>(&s_p0[wib][lane & 15]) + (lane >> 4);
   float* const p1 = reinterpret_cast<float*>(&s_p1[wib][lane & 15]) + (lane >> 4);
-  int nexcl = 0, curRep = 0;
+  int nexcl = 0, curRep = 0, tiles = 0;
   for (;;) {
     int L = 0;
     if (lane == 0) L = atomicAdd(a.workCounter, 1);
     L = __shfl_sync(0xffffffffu, L, 0);
     if (L >= a.numListsHost) break;
     const nbk_tile_list tl = a.lists[L];
-    if (tl.jtileEnd < tl.jtileStart) continue;  // warp-uniform
+    if (tl.jtileEnd < tl.jtileStart) {  // warp-uniform
+      if (lane == 0) a.listActive[L] = 0;
+      continue;
+    }
     float3 la = a.lata, lb = a.latb, lc = a.latc;
     if (a.compRep) {
       const int rep = __ldg(&a.compRep[tl.icompute]);
@@ -269,7 +245,6 @@ __global__ void __launch_bounds__(128) refineKernel(const __grid_constant__ Forc
       float4 xjNext = a.xyzq[jsNext + lane];
       int idxNext = a.atomIndex[jsNext + lane];
       for (int u = 0; u < nt; ++u) {
-        const int jt = jt0 + u;
         const int jstart = jsNext;
         float4 xj = xjNext;
         const int jIndex = idxNext;
@@ -322,15 +297,23 @@ __global__ void __launch_bounds__(128) refineKernel(const __grid_constant__ Forc
             }
           }
         }
-        a.tileExcls[jt].excl[lane] = blockOrder(mw, lane);
-        const bool any = __any_sync(0xffffffffu, mw != 0);
-        if (lane == 0) a.jtileActive[jt] = any ? 1 : 0;
-        activeTiles += any ? 1 : 0;
+        // tiles with listed pairs close up at the start of the list's slots
+        if (__any_sync(0xffffffffu, mw != 0)) {
+          const int slot = tl.jtileStart + activeTiles;
+          a.tileExcls[slot].excl[lane] = blockOrder(mw, lane);
+          if (lane == 0) a.tileJatomOut[slot] = jstart;
+          ++activeTiles;
+        }
         __syncwarp();
       }
     }
-    if (lane == 0) a.listActive[L] = activeTiles;
+    if (lane == 0) {
+      a.listActive[L] = activeTiles;
+      if (a.lenHist && activeTiles) atomicAdd(&a.lenHist[min(activeTiles, a.maxLen)], 1);
+    }
+    tiles += activeTiles;
   }
+  if (lane == 0 && tiles) atomicAdd(&a.counts[1], tiles);
   const int s = __reduce_add_sync(0xffffffffu, nexcl);
   if (lane == 0 && s) atomicAddFixed(&a.acc[(size_t)curRep * kAccCount + kAccNumExcl], (unsigned long long)s);
 }
@@ -353,72 +336,91 @@ cudaError_t launchRefine(const ForceArgs& a, int numSM, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The compacted lists in order of decreasing length (the order sortTileLists
+// The refined lists in order of decreasing length (the order sortTileLists
 // establishes, src/CudaTileListKernel.cu:1208-1600): with lists handed out
 // longest first from the work counter, the last lists to start are the
-// shortest, which trims the tail of the force launch (0.483 -> 0.448 ms at
-// 92k atoms). A counting sort over the lengths: histogram, offsets in
-// decreasing length, scatter. Lanes of a warp holding lists of the same
-// length combine their atomics (__match_any_sync), so popular lengths do not
-// serialise on one counter. Lists of equal length land in any order; nothing
-// computed from them depends on list order.
-__device__ __forceinline__ int listLength(const nbk_tile_list& t, int maxLen) {
-  return min(max(t.jtileEnd - t.jtileStart + 1, 0), maxLen);
-}
-
-__global__ void listLengthHistKernel(const nbk_tile_list* __restrict__ lists,
-                                     const int* __restrict__ numLists, int maxLen,
-                                     int* __restrict__ hist) {
-  const int n = *numLists;
-  const int lane = threadIdx.x & 31;
-  for (int L0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; L0 < n; L0 += gridDim.x * blockDim.x) {
-    const int L = L0 + lane;
-    const int len = L < n ? listLength(lists[L], maxLen) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, len);
-    if (len >= 0 && lane == __ffs(peers) - 1) atomicAdd(&hist[len], __popc(peers));
-  }
-}
-
-__global__ void listLengthScanKernel(int maxLen, int* __restrict__ hist) {
-  if (threadIdx.x != 0) return;
+// shortest, which trims the tail of the force launch. A counting sort over the
+// lengths that the refinement counted: offsets in decreasing length, scatter.
+// Lanes of a warp holding lists of the same length combine their atomics
+// (__match_any_sync), so popular lengths do not serialise on one counter.
+// Lists of equal length land in any order; nothing computed from them depends
+// on list order.
+// Descending offsets of the lengths 1..maxLen and the number of lists, by one
+// warp from the histogram that the refinement counted.
+__global__ void listLengthScanKernel(int maxLen, int* __restrict__ hist, int* __restrict__ counts) {
+  const int lane = threadIdx.x;
   int off = 0;
-  for (int len = maxLen; len >= 0; --len) {
-    const int c = hist[len];
-    hist[len] = off;
-    off += c;
+  for (int top = maxLen; top >= 1; top -= 32) {
+    const int len = top - lane;
+    const int c = len >= 1 ? hist[len] : 0;
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (len >= 1) hist[len] = off + incl - c;
+    off += __shfl_sync(0xffffffffu, incl, 31);
   }
+  if (lane == 0) counts[0] = off;
 }
 
-__global__ void listScatterKernel(const nbk_tile_list* __restrict__ src, const int* __restrict__ numLists,
-                                  int maxLen, int* __restrict__ cursor, nbk_tile_list* __restrict__ dst) {
-  const int n = *numLists;
+__global__ void listScatterKernel(int n, const nbk_tile_list* __restrict__ src,
+                                  const int* __restrict__ listActive, int maxLen,
+                                  int* __restrict__ cursor, nbk_tile_list* __restrict__ dst) {
   const int lane = threadIdx.x & 31;
   for (int L0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; L0 < n; L0 += gridDim.x * blockDim.x) {
     const int L = L0 + lane;
-    nbk_tile_list t;
-    int len = -1;
-    if (L < n) {
-      t = src[L];
-      len = listLength(t, maxLen);
-    }
+    const int tiles = L < n ? listActive[L] : 0;
+    const int len = min(tiles, maxLen);
     const unsigned peers = __match_any_sync(0xffffffffu, len);
     const int leader = __ffs(peers) - 1;
     int base = 0;
-    if (len >= 0 && lane == leader) base = atomicAdd(&cursor[len], __popc(peers));
+    if (len > 0 && lane == leader) base = atomicAdd(&cursor[len], __popc(peers));
     base = __shfl_sync(0xffffffffu, base, leader);
-    if (len >= 0) dst[base + __popc(peers & ((1u << lane) - 1u))] = t;
+    if (len > 0) {
+      nbk_tile_list t = src[L];
+      t.jtileEnd = t.jtileStart + tiles - 1;
+      dst[base + __popc(peers & ((1u << lane) - 1u))] = t;
+    }
   }
 }
 
-cudaError_t launchSortLists(int numListsMax, const nbk_tile_list* src, const int* numListsDev,
-                            int maxLen, int* hist, nbk_tile_list* dst, int numSM, cudaStream_t st) {
-  if (numListsMax <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * ((size_t)maxLen + 1), st);
-  if (e != cudaSuccess) return e;
-  const int blocks = min((numListsMax + 255) / 256, numSM * 4);
-  listLengthHistKernel<<<blocks, 256, 0, st>>>(src, numListsDev, maxLen, hist);
-  listLengthScanKernel<<<1, 32, 0, st>>>(maxLen, hist);
-  listScatterKernel<<<blocks, 256, 0, st>>>(src, numListsDev, maxLen, hist, dst);
+cudaError_t launchSortLists(int numLists, const nbk_tile_list* src, const int* listActive,
+                            int maxLen, int* hist, int* counts, nbk_tile_list* dst, int numSM,
+                            cudaStream_t st) {
+  if (numLists <= 0) return cudaSuccess;
+  const int blocks = min((numLists + 255) / 256, numSM * 4);
+  listLengthScanKernel<<<1, 32, 0, st>>>(maxLen, hist, counts);
+  listScatterKernel<<<blocks, 256, 0, st>>>(numLists, src, listActive, maxLen, hist, dst);
+  return cudaGetLastError();
+}
+
+// Export: list k's tiles from its own slots to the place in packed arrays that
+// dst[k] names, the masks from block order to the interface's (bit t of lane i
+// <-> j = (i + t) & 31). One warp per list.
+__global__ void exportTilesKernel(int numLists, const nbk_tile_list* __restrict__ lists,
+                                  const int* __restrict__ dst, const int* __restrict__ jatom,
+                                  const nbk_tile_excl* __restrict__ excl, int* __restrict__ jatomOut,
+                                  nbk_tile_excl* __restrict__ exclOut) {
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int L = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; L < numLists; L += warps) {
+    const int first = lists[L].jtileStart, n = lists[L].jtileEnd - first + 1, to = dst[L];
+    for (int k = 0; k < n; ++k) {
+      const unsigned row = blockOrder(excl[first + k].excl[lane], lane);
+      exclOut[to + k].excl[lane] = __funnelshift_r(row, row, lane);
+      if (lane == 0) jatomOut[to + k] = jatom[first + k];
+    }
+  }
+}
+
+cudaError_t launchExportTiles(int numLists, const nbk_tile_list* lists, const int* dst,
+                              const int* jatom, const nbk_tile_excl* excl, int* jatomOut,
+                              nbk_tile_excl* exclOut, cudaStream_t st) {
+  if (numLists <= 0) return cudaSuccess;
+  exportTilesKernel<<<min((numLists + 7) / 8, 4096), 256, 0, st>>>(numLists, lists, dst, jatom, excl,
+                                                                 jatomOut, exclOut);
   return cudaGetLastError();
 }
 
@@ -446,13 +448,10 @@ cudaError_t launchBuildLists(int numLists, const ListSeed* seeds,
 }
 
 cudaError_t launchCompact(int numLists, const nbk_tile_list* src, const int* listActive,
-                          const int* jtileActive, const int* jatomSrc, const nbk_tile_excl* exclSrc,
-                          nbk_tile_list* dst, int* jatomDst, nbk_tile_excl* exclDst, int* counters,
-                          int numSM, cudaStream_t st) {
+                          nbk_tile_list* dst, int* counters, int numSM, cudaStream_t st) {
   if (numLists <= 0) return cudaSuccess;
-  const int blocks = min((numLists + kCompactWarps - 1) / kCompactWarps, numSM * 8);
-  compactKernel<<<blocks, kCompactWarps * 32, 0, st>>>(numLists, src, listActive, jtileActive, jatomSrc,
-                                            exclSrc, dst, jatomDst, exclDst, counters);
+  const int blocks = min((numLists + kCompactThreads - 1) / kCompactThreads, numSM * 4);
+  compactKernel<<<blocks, kCompactThreads, 0, st>>>(numLists, src, listActive, dst, counters);
   return cudaGetLastError();
 }
 
