@@ -696,6 +696,9 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     r.tileJatomOut = h->jatom2.p;
     r.tileExcls = h->excl2.p;
     r.listActive = h->listActive.p;
+    r.lenHist = h->listsSorted ? h->lenHist.p : nullptr;
+    r.maxLen = h->maxListLen;
+    r.counts = h->counters.p;
     r.patchPairs = h->patchPairs.p;
     r.workCounter = h->counters.p + 3;
     // lists and tiles kept; with them the work counters of all three kernels
@@ -724,9 +727,6 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     a.liveOut = h->live.p;
   }
   NBK_CUDA(launchForce(a, flags, h->tuneMinBlocks[key], h->numSM, st), "force kernel");
-    r.lenHist = h->listsSorted ? h->lenHist.p : nullptr;
-    r.maxLen = h->maxListLen;
-    r.counts = h->counters.p;
   h->launches += 1;
   NBK_CUDA(timedEvent(h, kTimedMid, st), "timing event");
   const bool corrections = (flags & NBK_CORRECTIONS) && (h->numMod || h->numExc);
@@ -899,6 +899,13 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
     dExcl.release();
     NBK_CUDA(e, "export");
   }
+  if (tl)
+    for (int k = 0; k < cnt[0]; ++k) {
+      const int n = lists[k].jtileEnd - lists[k].jtileStart + 1;
+      lists[k].jtileStart = to[k];
+      lists[k].jtileEnd = to[k] + n - 1;
+      tl[k] = lists[k];
+    }
   return NBK_OK;
 }
 
@@ -932,13 +939,6 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
   NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int), st), "nbk_adjoint");
   AdjArgs a{};
   a.lists = h->refinedLists();
-  if (tl)
-    for (int k = 0; k < cnt[0]; ++k) {
-      const int n = lists[k].jtileEnd - lists[k].jtileStart + 1;
-      lists[k].jtileStart = to[k];
-      lists[k].jtileEnd = to[k] + n - 1;
-      tl[k] = lists[k];
-    }
   a.numListsDev = h->counters.p;
   a.tileJatomStart = h->jatom2.p;
   a.tileExcls = h->excl2.p;
