@@ -87,9 +87,11 @@ struct nbk_context {
   NbkConst c{};
   NbkConst64 c64{};
   PackedConst pk{};
+  DBuf<float4> forceTable;  // FP32 slow force factor (buildForceTable)
   int ljDim = 0;
   DBuf<float2> ljTable, ljExclTable;
   DBuf<double2> slowTable;  // FP64 phi_s rows (buildSlowTable)
+  DBuf<float4> adjTable;    // the same rows in FP32, padded to 8 (adjoint)
   int slowTableRows = 0;
   double slowStep = 2.0;
   DBuf<unsigned> exclBits;
@@ -381,6 +383,24 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   h->slowTableRows = buildSlowTable(p->ewaldcof, p->cutoff, p->pairlistdist, slow, &h->slowStep);
   fin(h->slowTable.ensure(slow.size() / 2), "nbk_create: alloc");
   if (rc == NBK_OK) fin(cudaMemcpy(h->slowTable.p, slow.data(), sizeof(double) * slow.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+  std::vector<float4> at(2 * (size_t)h->slowTableRows);
+  for (int k = 0; k < h->slowTableRows; ++k) {
+    const double* r = &slow[(size_t)k * kSlowTableRow];
+    at[2 * k] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
+    at[2 * k + 1] = make_float4((float)r[4], (float)r[5], 0.f, 0.f);
+  }
+  fin(h->adjTable.ensure(at.size()), "nbk_create: alloc");
+  if (rc == NBK_OK) fin(cudaMemcpy(h->adjTable.p, at.data(), sizeof(float4) * at.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+  std::vector<float4> ft;
+  double ftStep = 1.0;
+  h->pk.tabRows = buildForceTable(p->ewaldcof, p->cutoff, p->pairlistdist, ft, &ftStep);
+  h->pk.tabStep = (float)ftStep;  // a power of two
+  h->pk.tabInvStep = (float)(1.0 / ftStep);
+  if (h->pk.tabRows > 0) {
+    fin(h->forceTable.ensure(ft.size()), "nbk_create: alloc");
+    if (rc == NBK_OK) fin(cudaMemcpy(h->forceTable.p, ft.data(), sizeof(float4) * ft.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+    h->pk.tab = h->forceTable.p;
+  }
   fin(h->acc.ensure(kAccCount), "nbk_create: alloc");
   fin(h->counters.ensure(8), "nbk_create: alloc");
   fin(h->ve.ensure(1), "nbk_create: alloc");
@@ -400,6 +420,8 @@ NBK_API int nbk_destroy(nbk_handle h) {
   h->ljTable.release();
   h->ljExclTable.release();
   h->slowTable.release();
+  h->forceTable.release();
+  h->adjTable.release();
   h->exclBits.release();
   h->computes.release();
   h->vdwTypes.release();

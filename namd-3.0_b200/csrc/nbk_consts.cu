@@ -96,16 +96,17 @@ static double slowPhi(double beta, double rc, double s) {
   return (3.0 - s / (rc * rc)) / (2.0 * rc) - erfOverR(beta, s);
 }
 
-// One table of the given power-of-two step: row k the degree-5 Chebyshev
-// interpolant (6 nodes) on s in [k step - step/2, k step + step/2] written in
-// powers of w = s - k step. Returns the largest deviation from phi_s at 32
-// points per row between the nodes.
-static double fitSlowTable(double beta, double rc, double step, int rows, std::vector<double>& out) {
-  const int deg = kSlowTableDeg, nn = kSlowTableDeg + 1;
+// One table of the given power-of-two step: row k the Chebyshev interpolant of
+// degree deg (deg + 1 nodes) of f on s in [k step - step/2, k step + step/2]
+// written in powers of w = s - k step. Returns the largest deviation from f at
+// 32 points per row between the nodes.
+template <int deg, typename F>
+static double fitTable(const F& fun, double step, int rows, std::vector<double>& out) {
+  const int nn = deg + 1;
   const double half = 0.5 * step;
-  out.assign((size_t)rows * kSlowTableRow, 0.0);
+  out.assign((size_t)rows * nn, 0.0);
   // monomial coefficients of the Chebyshev polynomials T_0 .. T_deg
-  double T[kSlowTableDeg + 1][kSlowTableDeg + 1] = {};
+  double T[deg + 1][deg + 1] = {};
   T[0][0] = 1.0;
   T[1][1] = 1.0;
   for (int j = 2; j <= deg; ++j)
@@ -113,10 +114,10 @@ static double fitSlowTable(double beta, double rc, double step, int rows, std::v
   double worst = 0.0;
   for (int k = 0; k < rows; ++k) {
     const double centre = step * k;
-    double f[kSlowTableDeg + 1];
-    for (int m = 0; m < nn; ++m) f[m] = slowPhi(beta, rc, centre + half * std::cos(M_PI * (m + 0.5) / nn));
-    double* row = &out[(size_t)k * kSlowTableRow];
-    double cu[kSlowTableDeg + 1] = {};  // powers of u = w / half
+    double f[deg + 1];
+    for (int m = 0; m < nn; ++m) f[m] = fun(centre + half * std::cos(M_PI * (m + 0.5) / nn));
+    double* row = &out[(size_t)k * nn];
+    double cu[deg + 1] = {};  // powers of u = w / half
     for (int j = 0; j <= deg; ++j) {
       double cj = 0.0;
       for (int m = 0; m < nn; ++m) cj += f[m] * std::cos(j * M_PI * (m + 0.5) / nn);
@@ -129,7 +130,7 @@ static double fitSlowTable(double beta, double rc, double step, int rows, std::v
       const double w = half * (-1.0 + (q + 0.5) / 16.0);
       double p = row[deg];
       for (int m = deg - 1; m >= 0; --m) p = p * w + row[m];
-      worst = std::fmax(worst, std::fabs(p - slowPhi(beta, rc, centre + w)));
+      worst = std::fmax(worst, std::fabs(p - fun(centre + w)));
     }
   }
   return worst;
@@ -148,12 +149,57 @@ int buildSlowTable(double beta, double cutoff, double pairlistdist, std::vector<
   int rows = 0;
   for (;;) {
     rows = (int)std::ceil(smax / step + 0.5) + 1;
-    const double err = fitSlowTable(beta, cutoff, step, rows, out);
+    static_assert(kSlowTableRow == kSlowTableDeg + 1, "rows without padding");
+    const double err = fitTable<kSlowTableDeg>(
+        [&](double s) { return slowPhi(beta, cutoff, s); }, step, rows, out);
     if (err <= kSlowTableTol * scale || step <= kSlowTableStepMax / 128) break;
     step *= 0.5;
   }
   if (stepOut) *stepOut = step;
   return rows;
+}
+
+// (dE/dr)/r of the slow term per unit qq, 2 dphi_s/ds = (erf(x) - 2/sqrt(pi) x
+// e^{-x^2})/r^3 - 1/rc^3 with x = beta r: by its power series where it cancels.
+static double slowForceFactor(double beta, double rc, double s) {
+  const double rc3inv = 1.0 / (rc * rc * rc), y = beta * beta * s;
+  if (y < 0.5) {
+    // -2 d/ds of erfOverR's series
+    double term = 1.0, sum = 0.0;  // term: (-y)^(n-1)/(n-1)!
+    for (int n = 1; n < 80; ++n) {
+      sum += term / (2 * n + 1);
+      term *= -y / n;
+    }
+    return 4.0 * beta * beta * beta / std::sqrt(M_PI) * sum - rc3inv;
+  }
+  const double r = std::sqrt(s);
+  return (std::erf(beta * r) / r - 2.0 * beta / std::sqrt(M_PI) * std::exp(-y)) / s - rc3inv;
+}
+
+// The force kernel's FP32 table of the slow force factor over s in [0,
+// pairlistdist^2 + 2] (the runtime cutoff is at most the pairlist cutoff): the
+// step starts at 32 A^2 and is halved until the fit is within kForceTableTol of
+// the factor's largest value or the table would pass kForceTableMaxRows. Returns the
+// number of rows, 0 when the tolerance asks for more than that.
+int buildForceTable(double beta, double cutoff, double pairlistdist, std::vector<float4>& out,
+                    double* stepOut) {
+  const double smax = pairlistdist * pairlistdist + 2.0;
+  const double scale = std::fabs(slowForceFactor(beta, cutoff, 0.0)) + 1.0 / (cutoff * cutoff * cutoff);
+  std::vector<double> fit;
+  for (double step = kSlowTableStepMax;; step *= 0.5) {
+    const double need = std::ceil(smax / step + 0.5) + 1;
+    if (need > kForceTableMaxRows) return 0;
+    const int rows = (int)need;
+    if (fitTable<3>([&](double s) { return slowForceFactor(beta, cutoff, s); }, step, rows, fit) >
+        kForceTableTol * scale)
+      continue;
+    out.resize(rows);
+    for (int k = 0; k < rows; ++k)
+      out[k] = make_float4((float)fit[4 * k], (float)fit[4 * k + 1], (float)fit[4 * k + 2],
+                           (float)fit[4 * k + 3]);
+    *stepOut = step;
+    return rows;
+  }
 }
 
 }  // namespace nbk

@@ -36,6 +36,7 @@ constexpr int kForceWarps = 4;
 // parts hold whole groups), so every sum is independent of the split.
 constexpr int kFoldTiles = 4;
 constexpr int kForceThreads = kForceWarps * kWarp;
+constexpr size_t kForceTableBytes = 16 * 1024;  // slow force table copies per CTA
 
 // FP64 quantities of the precise pass; after a tile's pass lane q < kNumQ
 // holds quantity q: the fast and slow electrostatic energies, then the six
@@ -375,14 +376,16 @@ __device__ __forceinline__ float keepHalf(const float first, const float second,
 // work items (warps), contiguous parts of equal tile count. Both are launch
 // choices of the autotuner; results do not depend on them (fixed-point sums
 // per tile group).
-template <bool doEnergy, bool doVirial, bool doSlow, bool doBatch, int MINB>
+template <bool doEnergy, bool doVirial, bool doSlow, bool kTable, bool doBatch, int MINB>
 __global__ void __launch_bounds__(kForceThreads, MINB)
     forceKernel(const __grid_constant__ ForceArgs a) {
   // the live words feed the precise kernel, which runs on energy evaluations
   // and on virial evaluations with slow forces (it forms the slow virial)
   constexpr bool kLive = doEnergy || (doVirial && doSlow);
   constexpr int kNC = doSlow ? 6 : 3;  // force components: fast x y z, slow x y z
-  extern __shared__ __align__(16) float2 s_lj[];  // [ljDim*ljDim] (A, -B) (single system)
+  // the slow force table (kTable; a.tabCopies interleaved copies), then the LJ
+  // table [ljDim*ljDim] as (A, -B) (single system)
+  extern __shared__ __align__(16) float4 s_tab[];
   // the list's i atoms, shifted: (-x, -x, -y, -y), then (-z, -z, q, byte
   // offset of the type's LJ row)
   __shared__ float4 s_i[kForceWarps][2][kWarp];
@@ -408,14 +411,27 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
   const int li = lane & 7, lj = lane >> 3;
   const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
   const unsigned adrI = sharedAddr(&s_i[wib][0][li]), adrJ = sharedAddr(&s_j[wib][b2][0][lj]),
-                 adrT = sharedAddr(&s_jt[wib][b2][lj]), adrLJ = sharedAddr(s_lj);
+                 adrT = sharedAddr(&s_jt[wib][b2][lj]);
   const NbkConst& c = a.c;
   const int dim = c.ljDim;
+  const int tabEntries = kTable ? a.pk.tabRows * a.tabCopies : 0;
+  const unsigned adrLJ = sharedAddr(s_tab + tabEntries);
+  ForceTable T{};
+  if (kTable) {
+    for (int k = threadIdx.x; k < tabEntries; k += blockDim.x)
+      s_tab[k] = a.pk.tab[(unsigned)k / (unsigned)a.tabCopies];
+    T.stride = 16u * a.tabCopies;
+    T.base = sharedAddr(s_tab + (lane & (a.tabCopies - 1))) - kRowMagicBits * T.stride;
+    T.step = a.pk.tabStep;
+    T.invStep = a.pk.tabInvStep;
+    T.sMax = a.pk.tabStep * (float)(a.pk.tabRows - 1);
+  }
   if (!doBatch) {
+    float2* s_lj = reinterpret_cast<float2*>(s_tab + tabEntries);
     for (int k = threadIdx.x; k < dim * dim; k += blockDim.x)
       s_lj[k] = make_float2(a.ljTable[k].x, -a.ljTable[k].y);
-    __syncthreads();
   }
+  if (kTable || !doBatch) __syncthreads();
 
   const int numLists = a.numListsDev ? *a.numListsDev : a.numListsHost;
 
@@ -562,8 +578,8 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
           const float2 abB = doBatch ? __ldg((const float2*)(ljRow + tB)) : ldShared2(adrLJ + tB);
           const float2 QQ = make_float2(ib.z * jb.z, ib.z * jb.w);
           float2 F, FS, E;
-          pairForce2<doEnergy, doSlow>(R2, QQ, make_float2(abA.x, abB.x),
-                                       make_float2(abA.y, abB.y), a.pk, F, FS, E);
+          pairForce2<doEnergy, doSlow, kTable>(R2, QQ, make_float2(abA.x, abB.x),
+                                       make_float2(abA.y, abB.y), a.pk, T, F, FS, E);
           // an element that is no interacting pair may hold anything, NaN
           // included: it is replaced by an exact zero
           F = make_float2(aA ? F.x : 0.f, aB ? F.y : 0.f);
@@ -840,10 +856,23 @@ static cudaError_t launchPersistent(K kernel, OccCache& cache, int threads, size
 
 template <bool E, bool V, bool S, bool B, int MINB>
 static cudaError_t launchT(const ForceArgs& a, int numSM, cudaStream_t st) {
+  const size_t lj = B ? 0 : sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
+  if constexpr (S) {
+    if (a.pk.tabRows > 0) {
+      // as many copies of the table as fit in kForceTableBytes, up to the 8 that
+      // keep quarter warps free of bank conflicts
+      static OccCache cache;
+      ForceArgs t = a;
+      const size_t one = sizeof(float4) * (size_t)a.pk.tabRows;
+      t.tabCopies = 8;
+      while (t.tabCopies > 1 && one * t.tabCopies > kForceTableBytes) t.tabCopies /= 2;
+      return launchPersistent(forceKernel<E, V, S, true, B, MINB>, cache, kForceThreads,
+                              one * t.tabCopies + lj, numSM, st, t);
+    }
+  }
   static OccCache cache;
-  const size_t shmem = B ? 0 : sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
-  return launchPersistent(forceKernel<E, V, S, B, MINB>, cache, kForceThreads, shmem, numSM, st,
-                          a);
+  return launchPersistent(forceKernel<E, V, S, false, B, MINB>, cache, kForceThreads, lj, numSM,
+                          st, a);
 }
 
 template <bool E, bool V, bool S, bool B>

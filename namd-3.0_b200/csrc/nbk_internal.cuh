@@ -182,10 +182,32 @@ __device__ __forceinline__ double rsqrtApprox64(double x) {
 struct PackedConst {
   float2 dA, dB, hA;    // -12 c1 D, 12 c1, -6 c1 D
   float2 rc3inv;
-  float2 nBeta2Pi;      // -2 beta / sqrt(pi)
   float rc2, dMax;      // rc^2 (huge without switching), D
+  // the slow force factor: from its table (rows > 0), row k = (c0, c1, c2, c3)
+  // in w = s - k D, or from the erfc form
+  const float4* tab;
+  int tabRows;
+  float tabStep, tabInvStep;
+  float2 nBeta2Pi;      // -2 beta / sqrt(pi)
   float pBeta, gaussK;  // erfcShared's p times beta; exp(-beta^2 r^2) = 2^(gaussK r^2)
 };
+// The fit's error relative to the factor's largest value (at r = 0), and the
+// rows a table may have (16 KB of shared memory). At 3e-8 the fit is an order
+// below the rounding of the erfc form ((1 - erfc term) r^-3 cancels at short
+// range), and the benchmark's parameters give 93 rows.
+constexpr double kForceTableTol = 3e-8;
+constexpr int kForceTableMaxRows = 1024;
+
+// The table in shared memory, as a lane of the force kernel reads it: copies
+// interleaved row by row, so that with 8 of them the lanes of a quarter warp
+// read from 8 different bank groups whatever rows they want. A row's address
+// is base + bits(1.5 2^23 + row) * stride.
+struct ForceTable {
+  unsigned base, stride;
+  float step, invStep, sMax;
+};
+constexpr float kRowMagic = 12582912.0f;        // 1.5 2^23
+constexpr unsigned kRowMagicBits = 0x4B400000u;
 
 // FP32 pair math for two pairs (x and y elements); nB = -B. F, FS = (dE/dr)/r
 // of LJ + fast electrostatics and of the slow (PME real-space remainder)
@@ -197,16 +219,19 @@ struct PackedConst {
 // the LJ energy is formed here (doVdwEnergy; e6 = -6 E): the electrostatic
 // energies and the slow virial are formed in FP64 by the precise kernel
 // (nbk_force.cu). Callers replace the results of an element that is no
-// interacting pair. LJ is taken as r^-6 [(2 A r^-6 - B) (-6 S/r^2) + (A r^-6 -
-// B) (dS/dr)/r], which needs the fewest operations. The slow term regroups the
-// same quantities: with x = beta r, t = 1/(1 + p x) and e = exp(-x^2) =
-// 2^(gaussK r^2), erfc = t P(t) e and the force factor erfc + (2
-// beta/sqrt(pi)) r e = (t P(t) + (2 beta/sqrt(pi)) r) e; the bracket is formed
-// with its sign turned.
-template <bool doVdwEnergy, bool doSlow>
+// interacting pair (they may be anything, but their r^2 is clamped into the
+// table). LJ is taken as r^-6 [(2 A r^-6 - B) (-6 S/r^2) + (A r^-6 -
+// B) (dS/dr)/r], which needs the fewest operations. The slow factor (dE/dr)/r =
+// qq K(s) comes from the cubic table of K (kTable; 20 issue slots against 34 of
+// the erfc form, whose rcp and ex2 it saves, and a smaller error), or, when the
+// tolerance needs more rows than the table may have, from the erfc form: with
+// x = beta r, t = 1/(1 + p x) and e = exp(-x^2) = 2^(gaussK r^2), erfc = t P(t)
+// e and the force factor erfc + (2 beta/sqrt(pi)) r e = (t P(t) + (2
+// beta/sqrt(pi)) r) e; the bracket is formed with its sign turned.
+template <bool doVdwEnergy, bool doSlow, bool kTable>
 __device__ __forceinline__ void pairForce2(const float2 r2, const float2 qq, const float2 A,
-                                           const float2 nB, const PackedConst& c, float2& f,
-                                           float2& fs, float2& e6) {
+                                           const float2 nB, const PackedConst& c,
+                                           const ForceTable& T, float2& f, float2& fs, float2& e6) {
   const float2 rinv = make_float2(rsqrtApprox(r2.x), rsqrtApprox(r2.y));
   const float2 rinv2 = mul2(rinv, rinv);
   const float2 rinv3 = mul2(rinv, rinv2);
@@ -220,7 +245,17 @@ __device__ __forceinline__ void pairForce2(const float2 r2, const float2 qq, con
   const float2 lj = fma2(ab12, mul2(rinv2, s6), mul2(ab6, ds));
   f = fma2(lj, rinv6, mul2(qq, add2(c.rc3inv, neg2(rinv3))));
   if (doVdwEnergy) e6 = mul2(mul2(ab6, rinv6), s6);
-  if (doSlow) {
+  if (doSlow && kTable) {
+    // row = nearest integer to s/D, in the low bits of t
+    const float2 s = make_float2(fminf(r2.x, T.sMax), fminf(r2.y, T.sMax));
+    const float2 t = fma2(s, f2(T.invStep), f2(kRowMagic));
+    const float2 w = fma2(add2(t, f2(-kRowMagic)), f2(-T.step), s);
+    const float4 a = ldShared4(T.base + __float_as_uint(t.x) * T.stride);
+    const float4 b = ldShared4(T.base + __float_as_uint(t.y) * T.stride);
+    const float2 k = make_float2(fmaf(fmaf(fmaf(a.w, w.x, a.z), w.x, a.y), w.x, a.x),
+                                 fmaf(fmaf(fmaf(b.w, w.y, b.z), w.y, b.y), w.y, b.x));
+    fs = mul2(qq, k);
+  } else if (doSlow) {
     const float2 r = mul2(r2, rinv);
     const float2 t = make_float2(rcpApprox(fmaf(c.pBeta, r.x, 1.0f)),
                                  rcpApprox(fmaf(c.pBeta, r.y, 1.0f)));
@@ -334,6 +369,7 @@ struct ForceArgs {
   float3 lata, latb, latc;
   NbkConst c;
   PackedConst pk;              // force kernel
+  int tabCopies;               // copies of pk.tab in shared memory (set by the launch)
   long long* force;            // SoA [6][stride] fixed point
   int stride;
   long long* acc;              // [kAccCount]
