@@ -11,8 +11,9 @@
 //   dL/dx_j = dL/dd, dL/dx_i = -dL/dd
 //   dL/dqq = pF g_f + pS g_s + cE phi_f + cS phi_s
 //   dL/dA = pF gA + cV EA, dL/dB = pF gB + cV EB   (LJ is linear in A and B)
-// where ' = d/ds. The slow-term derivatives cancel to O(x) at small
-// x = beta r and are taken from their Taylor series there.
+// where ' = d/ds. The slow term comes from the FP64 table of phi_s (nbk_consts.cu)
+// rounded to FP32: g_s = 2 phi_s' and g_s' = 2 phi_s'' are the derivatives of a
+// row's polynomial, so nothing cancels at short range.
 #include "nbk_internal.cuh"
 #include "nbk_launch.h"
 
@@ -20,216 +21,283 @@ namespace nbk {
 
 constexpr int kAdjWarps = 4;
 constexpr int kAdjThreads = kAdjWarps * kWarp;
+constexpr int kAdjRow = 8;  // floats per row of the FP32 slow table (degree 5, padded)
+constexpr size_t kAdjTableBytes = 24 * 1024;  // most shared memory the table's copies take
+static_assert(kSlowTableDeg == 5, "slow rows of six coefficients");
 
-// Slow (PME real-space) electrostatics per unit qq, as functions of s = r^2:
-//   g_s  = -1/rc^3 + beta^3 J(x),  J = (erf x - 2/sqrt(pi) x e^{-x^2}) / x^3
-//   g_s' = beta^5 K(x),            K = e^{-x^2}(2/x^2 + 3/x^4)/sqrt(pi) - 1.5 erf(x)/x^5
-//   phi_s = h(s) - erf(x)/r
-__device__ __forceinline__ void slowTerms(float r, float rinv, float x, float beta, float rc3inv,
-                                          float h, float& gs, float& dgs, float& phis) {
-  const float y = x * x;
-  const float ex = __expf(-y);
-  const float erfc_ = erfcShared(x, ex);
-  const float erfx = 1.0f - erfc_;
-  const float b2 = beta * beta, b3 = b2 * beta, b5 = b3 * b2;
-  float J, K;
-  if (x < 0.7f) {
-    // J = 2/sqrt(pi) sum_{n>=1} (-1)^{n+1} 2n y^{n-1} / ((2n+1) n!)
-    float q = 14.0f / (15.0f * 5040.0f);  // n = 7
-    q = fmaf(q, -y, 12.0f / (13.0f * 720.0f));
-    q = fmaf(q, -y, 10.0f / (11.0f * 120.0f));
-    q = fmaf(q, -y, 8.0f / (9.0f * 24.0f));
-    q = fmaf(q, -y, 6.0f / (7.0f * 6.0f));
-    q = fmaf(q, -y, 4.0f / (5.0f * 2.0f));
-    q = fmaf(q, -y, 2.0f / 3.0f);
-    J = 1.1283791671f * q;
-    // K = 1/sqrt(pi) sum_{m>=2} (-1)^m 4m(1-m) / (m! (2m+1)) y^{m-2}
-    float k = -4.0f * 10.0f * 9.0f / (3628800.0f * 21.0f);           // m = 10
-    k = fmaf(k, y, 4.0f * 9.0f * 8.0f / (362880.0f * 19.0f));        // m = 9
-    k = fmaf(k, y, -4.0f * 8.0f * 7.0f / (40320.0f * 17.0f));        // m = 8
-    k = fmaf(k, y, 4.0f * 7.0f * 6.0f / (5040.0f * 15.0f));          // m = 7
-    k = fmaf(k, y, -4.0f * 6.0f * 5.0f / (720.0f * 13.0f));          // m = 6
-    k = fmaf(k, y, 4.0f * 5.0f * 4.0f / (120.0f * 11.0f));           // m = 5
-    k = fmaf(k, y, -4.0f * 4.0f * 3.0f / (24.0f * 9.0f));            // m = 4
-    k = fmaf(k, y, 4.0f * 3.0f * 2.0f / (6.0f * 7.0f));              // m = 3
-    k = fmaf(k, y, -4.0f * 2.0f * 1.0f / (2.0f * 5.0f));             // m = 2
-    K = 0.5641895835f * k;
-  } else {
-    const float xi = 1.0f / x, xi2 = xi * xi, xi3 = xi2 * xi;
-    J = (erfx - 1.1283791671f * x * ex) * xi3;
-    K = 0.5641895835f * ex * (2.0f + 3.0f * xi2) * xi2 - 1.5f * erfx * xi3 * xi2;
-  }
-  gs = fmaf(b3, J, -rc3inv);
-  dgs = b5 * K;
-  phis = h - erfx * rinv;
-  (void)r;
+// phi_s, phi_s' and phi_s'' of one pair from its table row.
+struct SlowRow {
+  float phi, d1, d2;
+};
+__device__ __forceinline__ SlowRow slowRow(const float4 a, const float4 b, const float w) {
+  SlowRow r;
+  r.phi = fmaf(fmaf(fmaf(fmaf(fmaf(b.y, w, b.x), w, a.w), w, a.z), w, a.y), w, a.x);
+  r.d1 = fmaf(fmaf(fmaf(fmaf(5.0f * b.y, w, 4.0f * b.x), w, 3.0f * a.w), w, 2.0f * a.z), w, a.y);
+  r.d2 = fmaf(fmaf(fmaf(20.0f * b.y, w, 12.0f * b.x), w, 6.0f * a.w), w, 2.0f * a.z);
+  return r;
 }
 
+// Adds (x, y) to a pair of sums in shared memory: one 64-bit compare-and-swap
+// for both, where two FP32 shared atomics would be two such loops.
+__device__ __forceinline__ void atomicAddPair(float2* p, const float x, const float y) {
+  unsigned long long* u = reinterpret_cast<unsigned long long*>(p);
+  unsigned long long old = *reinterpret_cast<volatile unsigned long long*>(u), seen;
+  do {
+    seen = old;
+    const float2 v = make_float2(__uint_as_float((unsigned)seen) + x,
+                                 __uint_as_float((unsigned)(seen >> 32)) + y);
+    old = atomicCAS(u, seen,
+                    (unsigned long long)__float_as_uint(v.x) |
+                        ((unsigned long long)__float_as_uint(v.y) << 32));
+  } while (old != seen);
+}
 
-
-template <bool doSlow>
-__global__ void __launch_bounds__(kAdjThreads, 6) adjointKernel(const __grid_constant__ AdjArgs a) {
-  extern __shared__ float s_dyn[];  // s_lj (float2[dim^2]) then s_gAB (float[2 dim^2])
-  __shared__ float4 s_x[kAdjWarps][kWarp];
-  __shared__ float4 s_wf[kAdjWarps][kWarp];
-  __shared__ float4 s_ws[kAdjWarps][kWarp];
-  __shared__ int s_t[kAdjWarps][kWarp];
+// One warp per tile list, a tile as 16 blocks of 8 x 8 atoms as in the force
+// kernel (two j atoms per lane through packed FP32, i and j sums in registers
+// over a list and over a row of blocks). The kernel is bound by issue slots;
+// by diagonals of the tile, one pair per lane and step with the j sums rotated
+// between steps, it took 410 us at 24,000 atoms.
+template <bool doSlow, bool kShared>
+__global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_constant__ AdjArgs a) {
+  // the slow table's copies (kShared), the LJ table (A, -B), the LJ gradients
+  extern __shared__ __align__(16) float4 s_dyn[];
+  // i atoms: (-x, -x, -y, -y), (-z, -z, q, type), wF and wS as (x, x, y, y),
+  // (Fz, Fz, Sz, Sz), (Sx, Sx, Sy, Sy)
+  __shared__ float4 s_i[kAdjWarps][5][kWarp];
+  // j atoms by pairs (j, j + 4), two copies in turned order as in the force
+  // kernel: (x, x', y, y'), (z, z', q, q'), -wF and -wS likewise; types
+  __shared__ float4 s_j[kAdjWarps][2][5][16];
+  __shared__ float2 s_jt[kAdjWarps][2][16];
   const NbkConst& c = a.c;
+  const PackedConst& k = a.pk;
   const int dim = c.ljDim, d2 = dim * dim;
-  float2* s_lj = reinterpret_cast<float2*>(s_dyn);
-  float* s_gA = s_dyn + 2 * d2;
-  float* s_gB = s_gA + d2;
-  for (int k = threadIdx.x; k < d2; k += blockDim.x) {
-    s_lj[k] = a.ljTable[k];
-    s_gA[k] = 0.0f;
-    s_gB[k] = 0.0f;
+  const int tabEntries = kShared ? 2 * a.slowRows * a.tabCopies : 0;
+  float2* s_lj = reinterpret_cast<float2*>(s_dyn + tabEntries);
+  float2* s_g = s_lj + d2;
+  for (int m = threadIdx.x; m < tabEntries; m += blockDim.x)
+    s_dyn[m] = a.slowTable[(unsigned)m / (unsigned)a.tabCopies];
+  for (int m = threadIdx.x; m < d2; m += blockDim.x) {
+    s_lj[m] = make_float2(a.ljTable[m].x, -a.ljTable[m].y);
+    s_g[m] = make_float2(0.f, 0.f);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int li = lane & 7, lj = lane >> 3;
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
+  const unsigned adrI = sharedAddr(&s_i[wib][0][li]), adrJ = sharedAddr(&s_j[wib][b2][0][lj]),
+                 adrT = sharedAddr(&s_jt[wib][b2][lj]), adrLJ = sharedAddr(s_lj),
+                 stride = 16u * a.tabCopies,
+                 adrTab = sharedAddr(s_dyn + (lane & (a.tabCopies - 1))) - kRowMagicBits * 2u * stride;
+  const float sMax = a.slowStep * (float)(a.slowRows - 1);
   const int numLists = *a.numListsDev;
   for (;;) {
-    int L = 0;
-    if (lane == 0) L = atomicAdd(a.workCounter, 1);
-    L = __shfl_sync(0xffffffffu, L, 0);
+    const int L = drawItem(a.workCounter, lane);
     if (L >= numLists) break;
     const nbk_tile_list tl = a.lists[L];
-    if (tl.jtileEnd < tl.jtileStart) continue;
     const float3 sh = shiftOf(make_float3(tl.offsetXYZ.x, tl.offsetXYZ.y, tl.offsetXYZ.z), a.lata,
                               a.latb, a.latc);
     const int iatom = tl.iatomStart + lane;
-    float4 xi = a.xyzq[iatom];
-    xi.x = __fadd_rn(xi.x, sh.x);
-    xi.y = __fadd_rn(xi.y, sh.y);
-    xi.z = __fadd_rn(xi.z, sh.z);
-    const int tiRaw = a.vdwTypes[iatom];
-    const int ti = tiRaw * dim;
-    const bool mi = a.typeMask[tiRaw] != 0;
-    const float4 wfi = a.wF[iatom];
-    const float4 wsi = doSlow ? a.wS[iatom] : make_float4(0.f, 0.f, 0.f, 0.f);
-    float gix = 0.f, giy = 0.f, giz = 0.f, giq = 0.f;
+    // byte offsets of types in the tables; bit 0 marks a type whose LJ gradients are wanted
+    {
+      const float4 xi = a.xyzq[iatom], wf = a.wF[iatom];
+      const float4 ws = doSlow ? a.wS[iatom] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const int ty = a.vdwTypes[iatom];
+      const float x = -__fadd_rn(xi.x, sh.x), y = -__fadd_rn(xi.y, sh.y), z = -__fadd_rn(xi.z, sh.z);
+      const int off = ty * dim * 8 + (a.typeMask[ty] != 0 ? 1 : 0);
+      s_i[wib][0][lane] = make_float4(x, x, y, y);
+      s_i[wib][1][lane] = make_float4(z, z, xi.w, __int_as_float(off));
+      s_i[wib][2][lane] = make_float4(wf.x, wf.x, wf.y, wf.y);
+      s_i[wib][3][lane] = make_float4(wf.z, wf.z, ws.z, ws.z);
+      s_i[wib][4][lane] = make_float4(ws.x, ws.x, ws.y, ws.y);
+    }
+    float gi[4][4];  // sums of v (= -dL/dx_i) and of q_j dL/dqq for the atoms 8 I + li
+#pragma unroll
+    for (int I = 0; I < 4; ++I) gi[I][0] = gi[I][1] = gi[I][2] = gi[I][3] = 0.f;
     for (int jt = tl.jtileStart; jt <= tl.jtileEnd; ++jt) {
-      // from block order to rows (bit j of lane i), then bit t <-> j = (lane + t) & 31
-      const unsigned rowMask = blockOrder(a.tileExcls[jt].excl[lane], lane);
-      const unsigned mask = __funnelshift_r(rowMask, rowMask, lane);
-      unsigned stepMask = __reduce_or_sync(0xffffffffu, mask);
-      if (!stepMask) continue;
+      const unsigned mask = a.tileExcls[jt].excl[lane];  // block order
       const int jstart = a.tileJatomStart[jt];
-      s_x[wib][lane] = a.xyzq[jstart + lane];
-      s_wf[wib][lane] = a.wF[jstart + lane];
-      if (doSlow) s_ws[wib][lane] = a.wS[jstart + lane];
-      s_t[wib][lane] = a.vdwTypes[jstart + lane];
-      __syncwarp();
-      float gjx = 0.f, gjy = 0.f, gjz = 0.f, gjq = 0.f;
-      int tPrev = 0;
-      while (stepMask) {
-        const int t = __ffs(stepMask) - 1;
-        stepMask &= stepMask - 1;
-        const int delta = t - tPrev;
-        if (delta) {
-          const int src = (lane + delta) & 31;
-          gjx = __shfl_sync(0xffffffffu, gjx, src);
-          gjy = __shfl_sync(0xffffffffu, gjy, src);
-          gjz = __shfl_sync(0xffffffffu, gjz, src);
-          gjq = __shfl_sync(0xffffffffu, gjq, src);
-        }
-        tPrev = t;
-        const int j = (lane + t) & 31;
-        const float4 xj = s_x[wib][j];
-        const float dx = __fsub_rn(xj.x, xi.x), dy = __fsub_rn(xj.y, xi.y), dz = __fsub_rn(xj.z, xi.z);
-        const float r2 = dist2(dx, dy, dz);
-        if (((mask >> t) & 1u) && r2 < c.cutoff2) {
-          const float4 wfj = s_wf[wib][j];
-          const float ufx = wfi.x - wfj.x, ufy = wfi.y - wfj.y, ufz = wfi.z - wfj.z;
-          const float pF = fmaf(ufz, dz, fmaf(ufy, dy, ufx * dx));
-          float usx = 0.f, usy = 0.f, usz = 0.f, pS = 0.f;
-          if (doSlow) {
-            const float4 wsj = s_ws[wib][j];
-            usx = wsi.x - wsj.x;
-            usy = wsi.y - wsj.y;
-            usz = wsi.z - wsj.z;
-            pS = fmaf(usz, dz, fmaf(usy, dy, usx * dx));
-          }
-          const int tj = s_t[wib][j];
-          const float2 ab = s_lj[ti + tj];
-          const float rinv = rsqrtf(r2);
-          const float si = rinv * rinv;               // 1/s
-          const float s3 = si * si * si, s6 = s3 * s3;
-          // LJ: W = A s^-6 - B s^-3 and its s-derivatives; switch S(s)
-          const float WA1 = -6.0f * s6 * si, WB1 = 3.0f * s3 * si;
-          const float WA2 = 42.0f * s6 * si * si, WB2 = -12.0f * s3 * si * si;
-          float S = 1.0f, S1 = 0.0f, S2 = 0.0f;
-          if (c.switching) {
-            const float t2 = fmaxf(r2, c.rs2);
-            const float dd = c.rc2 - t2;
-            // lj0..lj3 carry c1 = 1/(rc2-rs2)^3
-            S = dd * dd * fmaf(c.lj1, t2, c.lj0);
-            S1 = 0.5f * dd * fmaf(c.lj2, t2, c.lj3);  // 6 c1 (rc2-s)(rs2-s)
-            // S'' = 6 c1 (2s - rs2 - rc2) above rs, 0 below (lj1 = 2 c1)
-            S2 = (r2 > c.rs2) ? c.lj1 * (6.0f * t2 - 3.0f * c.rs2 - 3.0f * c.rc2) : 0.0f;
-          }
-          const float gA = 2.0f * fmaf(WA1, S, s6 * S1);
-          const float gB = 2.0f * fmaf(WB1, S, -s3 * S1);
-          const float glj = fmaf(ab.x, gA, ab.y * gB);
-          const float dglj = 2.0f * (ab.x * fmaf(WA2, S, fmaf(2.0f * WA1, S1, s6 * S2)) +
-                                     ab.y * fmaf(WB2, S, fmaf(2.0f * WB1, S1, -s3 * S2)));
-          const float qi = xi.w, qj = xj.w, qq = qi * qj;
-          const float rinv3 = rinv * si;
-          const float gf = c.rc3inv - rinv3;
-          const float dgf = 1.5f * rinv3 * si;
-          const float h = fmaf(c.hB, r2, c.hA);
-          const float phif = rinv - h;
-          float gs = 0.f, dgs = 0.f, phis = 0.f;
-          if (doSlow) slowTerms(r2 * rinv, rinv, c.beta * r2 * rinv, c.beta, c.rc3inv, h, gs, dgs, phis);
-          const float g = fmaf(qq, gf, glj);
-          const float radial = 2.0f * fmaf(pF, fmaf(qq, dgf, dglj), pS * qq * dgs) +
-                               fmaf(a.cV, glj, qq * fmaf(a.cE, gf, a.cS * gs));
-          const float gsq = qq * gs;
-          const float vx = fmaf(radial, dx, fmaf(g, ufx, gsq * usx));
-          const float vy = fmaf(radial, dy, fmaf(g, ufy, gsq * usy));
-          const float vz = fmaf(radial, dz, fmaf(g, ufz, gsq * usz));
-          gjx += vx;
-          gjy += vy;
-          gjz += vz;
-          gix -= vx;
-          giy -= vy;
-          giz -= vz;
-          const float dqq = fmaf(pF, gf, fmaf(pS, gs, fmaf(a.cE, phif, a.cS * phis)));
-          giq = fmaf(qj, dqq, giq);
-          gjq = fmaf(qi, dqq, gjq);
-          if (mi || a.typeMask[tj]) {
-            const float EA = s6 * S, EB = -s3 * S;
-            atomicAdd(&s_gA[ti + tj], fmaf(pF, gA, a.cV * EA));
-            atomicAdd(&s_gB[ti + tj], fmaf(pF, gB, a.cV * EB));
-          }
-        }
-      }
       {
-        const int src = (lane + (32 - tPrev)) & 31;
-        gjx = __shfl_sync(0xffffffffu, gjx, src);
-        gjy = __shfl_sync(0xffffffffu, gjy, src);
-        gjz = __shfl_sync(0xffffffffu, gjz, src);
-        gjq = __shfl_sync(0xffffffffu, gjq, src);
+        const float4 xj = a.xyzq[jstart + lane], wf = a.wF[jstart + lane];
+        const float4 ws = doSlow ? a.wS[jstart + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int ty = a.vdwTypes[jstart + lane];
+        const int off = ty * 8 + (a.typeMask[ty] != 0 ? 1 : 0);
+        const int m = (lane >> 3) * 4 + (lane & 3), e = (lane >> 2) & 1;
+#pragma unroll
+        for (int copy = 0; copy < 2; ++copy) {
+          const int ec = copy ? 1 - e : e;
+          float* p = reinterpret_cast<float*>(&s_j[wib][copy][0][m]) + ec;
+          p[0] = xj.x;
+          p[2] = xj.y;
+          p[64] = xj.z;
+          p[66] = xj.w;
+          p[128] = -wf.x;
+          p[130] = -wf.y;
+          p[192] = -wf.z;
+          p[194] = -ws.z;
+          p[256] = -ws.x;
+          p[258] = -ws.y;
+          reinterpret_cast<int*>(&s_jt[wib][copy][m])[ec] = off;
+        }
       }
-      const int jatom = jstart + lane;
-      if (gjx != 0.f || gjy != 0.f || gjz != 0.f || gjq != 0.f) {
-        atomicAddFixed(&a.grad[0 * (size_t)a.stride + jatom], toFixedForce(gjx));
-        atomicAddFixed(&a.grad[1 * (size_t)a.stride + jatom], toFixedForce(gjy));
-        atomicAddFixed(&a.grad[2 * (size_t)a.stride + jatom], toFixedForce(gjz));
-        atomicAddFixed(&a.grad[3 * (size_t)a.stride + jatom], toFixedForce(gjq));
+      unsigned todo = __reduce_or_sync(0xffffffffu, mask);
+      __syncwarp();
+#pragma unroll 1
+      while (todo) {  // live rows of blocks (warp-uniform)
+        const int J8 = (__ffs(todo) - 1) & 24;
+        const unsigned rowAny = (todo >> J8) & 0xffu;
+        todo &= ~(0xffu << J8);
+        const unsigned mrow = mask >> J8;
+        const unsigned aj = adrJ + J8 * 8;
+        const float4 j0 = ldShared4(aj), j1 = ldShared4(aj + 256), j2 = ldShared4(aj + 512),
+                     j3 = ldShared4(aj + 768);
+        const float4 j4 = doSlow ? ldShared4(aj + 1024) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float2 tj = ldShared2(adrT + J8 * 4);
+        const float2 QJ = make_float2(j1.z, j1.w);
+        float2 gj[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gj[q] = f2(0.f);
+#pragma unroll
+        for (int I = 0; I < 4; ++I) {
+          if (!(rowAny & (0x11u << I))) continue;  // warp-uniform
+          const unsigned ai = adrI + 128 * I;
+          const float4 i0 = ldShared4(ai), i1 = ldShared4(ai + 512);
+          const float2 DX = add2(make_float2(j0.x, j0.y), make_float2(i0.x, i0.y)),
+                       DY = add2(make_float2(j0.z, j0.w), make_float2(i0.z, i0.w)),
+                       DZ = add2(make_float2(j1.x, j1.y), make_float2(i1.x, i1.y));
+          const float2 R2 = fma2(DZ, DZ, fma2(DX, DX, mul2(DY, DY)));  // dist2's order
+          const bool aA = (mrow & (1u << I)) && (R2.x < c.cutoff2);
+          const bool aB = (mrow & (0x10u << I)) && (R2.y < c.cutoff2);
+          if (!__any_sync(0xffffffffu, aA || aB)) continue;
+          const float4 i2 = ldShared4(ai + 1024), i3 = ldShared4(ai + 1536);
+          const float2 UX = add2(make_float2(i2.x, i2.y), make_float2(j2.x, j2.y)),
+                       UY = add2(make_float2(i2.z, i2.w), make_float2(j2.z, j2.w)),
+                       UZ = add2(make_float2(i3.x, i3.y), make_float2(j3.x, j3.y));
+          const float2 pF = fma2(UZ, DZ, fma2(UY, DY, mul2(UX, DX)));
+          const int tA = __float_as_int(i1.w) + __float_as_int(tj.x),
+                    tB = __float_as_int(i1.w) + __float_as_int(tj.y);
+          const float2 abA = ldShared2(adrLJ + (tA & ~7)), abB = ldShared2(adrLJ + (tB & ~7));
+          const float2 A = make_float2(abA.x, abB.x), nB = make_float2(abA.y, abB.y);
+          const float2 rinv = make_float2(rsqrtApprox(R2.x), rsqrtApprox(R2.y));
+          const float2 si = mul2(rinv, rinv);  // 1/s
+          const float2 rinv3 = mul2(rinv, si);
+          const float2 s3 = mul2(mul2(si, si), si), s6 = mul2(s3, s3);
+          // the switch S and its derivatives in s: with d and T as at
+          // PackedConst, S = -(d (T - 6 c1 D d))/6, S' = T/2, S'' = 6 c1 (D - 2 d)
+          // beyond rs, 0 below
+          const float2 drs = make_float2(k.rc2 - R2.x, k.rc2 - R2.y);
+          const float2 dd = make_float2(fminf(drs.x, k.dMax), fminf(drs.y, k.dMax));
+          const float2 TT = mul2(dd, fma2(k.dB, dd, k.dA));
+          const float2 S = mul2(mul2(dd, fma2(k.hA, dd, TT)), f2(-1.0f / 6.0f));
+          const float2 S1 = mul2(TT, f2(0.5f));
+          const float2 S2r = fma2(mul2(k.dB, f2(-1.0f)), dd, neg2(k.hA));
+          const float2 S2 = make_float2(drs.x < k.dMax ? S2r.x : 0.f, drs.y < k.dMax ? S2r.y : 0.f);
+          // LJ, E = A s^-6 S - B s^-3 S: gA, gB = 2 d/ds per unit A, -B, and g_lj'
+          const float2 m = mul2(si, S);
+          const float2 gA = mul2(s6, fma2(f2(-12.0f), m, TT));
+          const float2 gnB = mul2(s3, fma2(f2(-6.0f), m, TT));
+          const float2 glj = fma2(A, gA, mul2(nB, gnB));
+          const float2 hA = mul2(s6, fma2(si, fma2(f2(42.0f), m, mul2(f2(-12.0f), S1)), S2));
+          const float2 hB = mul2(s3, fma2(si, fma2(f2(12.0f), m, mul2(f2(-6.0f), S1)), S2));
+          const float2 hlj = fma2(A, hA, mul2(nB, hB));  // g_lj' / 2
+          const float2 qi = f2(i1.z), qq = mul2(qi, QJ);
+          const float2 gf = add2(k.rc3inv, neg2(rinv3));
+          const float2 hf = mul2(f2(0.75f), mul2(rinv3, si));  // g_f' / 2
+          const float2 phif = add2(rinv, neg2(fma2(f2(c.hB), R2, f2(c.hA))));
+          const float2 g = fma2(qq, gf, glj);
+          // radial: 2 (pF g' + pS gs') + cV g_lj + cE qq g_f + cS qq g_s
+          float2 rad = fma2(mul2(pF, f2(4.0f)), fma2(qq, hf, hlj), mul2(f2(a.cV), glj));
+          float2 qr = mul2(f2(a.cE), gf);
+          float2 dqq = fma2(pF, gf, mul2(f2(a.cE), phif));
+          float2 VX = mul2(g, UX), VY = mul2(g, UY), VZ = mul2(g, UZ);
+          if constexpr (doSlow) {
+            const float4 i4 = ldShared4(ai + 2048);
+            const float2 WX = add2(make_float2(i4.x, i4.y), make_float2(j4.x, j4.y)),
+                         WY = add2(make_float2(i4.z, i4.w), make_float2(j4.z, j4.w)),
+                         WZ = add2(make_float2(i3.z, i3.w), make_float2(j3.z, j3.w));
+            const float2 pS = fma2(WZ, DZ, fma2(WY, DY, mul2(WX, DX)));
+            const float2 sc = make_float2(fminf(R2.x, sMax), fminf(R2.y, sMax));
+            const float2 t = fma2(sc, f2(a.slowInvStep), f2(kRowMagic));
+            const float2 w = fma2(add2(t, f2(-kRowMagic)), f2(-a.slowStep), sc);
+            SlowRow ra, rb;
+            if constexpr (kShared) {
+              const unsigned pa = adrTab + __float_as_uint(t.x) * 2u * stride,
+                             pb = adrTab + __float_as_uint(t.y) * 2u * stride;
+              ra = slowRow(ldShared4(pa), ldShared4(pa + stride), w.x);
+              rb = slowRow(ldShared4(pb), ldShared4(pb + stride), w.y);
+            } else {
+              const float4* pa = a.slowTable + 2 * (size_t)(__float_as_uint(t.x) - kRowMagicBits);
+              const float4* pb = a.slowTable + 2 * (size_t)(__float_as_uint(t.y) - kRowMagicBits);
+              ra = slowRow(__ldg(pa), __ldg(pa + 1), w.x);
+              rb = slowRow(__ldg(pb), __ldg(pb + 1), w.y);
+            }
+            const float2 gs = make_float2(2.0f * ra.d1, 2.0f * rb.d1);
+            const float2 d2s = make_float2(ra.d2, rb.d2);  // gs' / 2
+            const float2 phis = make_float2(ra.phi, rb.phi);
+            rad = fma2(mul2(pS, f2(4.0f)), mul2(qq, d2s), rad);
+            qr = fma2(f2(a.cS), gs, qr);
+            dqq = fma2(pS, gs, fma2(f2(a.cS), phis, dqq));
+            float2 gq = mul2(qq, gs);
+            gq = make_float2(aA ? gq.x : 0.f, aB ? gq.y : 0.f);
+            VX = fma2(gq, WX, make_float2(aA ? VX.x : 0.f, aB ? VX.y : 0.f));
+            VY = fma2(gq, WY, make_float2(aA ? VY.x : 0.f, aB ? VY.y : 0.f));
+            VZ = fma2(gq, WZ, make_float2(aA ? VZ.x : 0.f, aB ? VZ.y : 0.f));
+          } else {
+            VX = make_float2(aA ? VX.x : 0.f, aB ? VX.y : 0.f);
+            VY = make_float2(aA ? VY.x : 0.f, aB ? VY.y : 0.f);
+            VZ = make_float2(aA ? VZ.x : 0.f, aB ? VZ.y : 0.f);
+          }
+          rad = fma2(qq, qr, rad);
+          // an element that is no interacting pair may hold anything: exact zeros
+          rad = make_float2(aA ? rad.x : 0.f, aB ? rad.y : 0.f);
+          dqq = make_float2(aA ? dqq.x : 0.f, aB ? dqq.y : 0.f);
+          VX = fma2(rad, DX, VX);
+          VY = fma2(rad, DY, VY);
+          VZ = fma2(rad, DZ, VZ);
+          gi[I][0] += VX.x + VX.y;
+          gi[I][1] += VY.x + VY.y;
+          gi[I][2] += VZ.x + VZ.y;
+          gi[I][3] = fmaf(QJ.y, dqq.y, fmaf(QJ.x, dqq.x, gi[I][3]));
+          gj[0] = add2(gj[0], VX);
+          gj[1] = add2(gj[1], VY);
+          gj[2] = add2(gj[2], VZ);
+          gj[3] = fma2(qi, dqq, gj[3]);
+          // dL/dA = pF gA + cV s^-6 S, dL/dB = -(pF gnB + cV s^-3 S)
+          const float2 cS6 = mul2(f2(a.cV), S);
+          const float2 LA = fma2(pF, gA, mul2(cS6, s6)), LB = neg2(fma2(pF, gnB, mul2(cS6, s3)));
+          const int ti = __float_as_int(i1.w);
+          const bool wA = aA && ((ti | __float_as_int(tj.x)) & 1),
+                     wB = aB && ((ti | __float_as_int(tj.y)) & 1);
+          if (wA) atomicAddPair(s_g + (tA >> 3), LA.x, LB.x);
+          if (wB) atomicAddPair(s_g + (tB >> 3), LA.y, LB.y);
+        }
+        // the row's sums over the eight i lanes; lane bits 1 and 0 keep one of
+        // the components x, y, z, q of the lane's j atom
+        float u[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[q] = gj[q].x + __shfl_xor_sync(0xffffffffu, gj[q].y, 4);
+        const float lo = keepHalf(u[0], u[2], b1, 2), hi = keepHalf(u[1], u[3], b1, 2);
+        const float v = keepHalf(lo, hi, b0, 1);
+        if (v != 0.f)
+          atomicAddFixed(&a.grad[(size_t)((b1 ? 2 : 0) + (b0 ? 1 : 0)) * a.stride + jstart + J8 +
+                                 (lane & 4) + lj],
+                         toFixedForce(v));
       }
       __syncwarp();
     }
-    if (gix != 0.f || giy != 0.f || giz != 0.f || giq != 0.f) {
-      atomicAddFixed(&a.grad[0 * (size_t)a.stride + iatom], toFixedForce(gix));
-      atomicAddFixed(&a.grad[1 * (size_t)a.stride + iatom], toFixedForce(giy));
-      atomicAddFixed(&a.grad[2 * (size_t)a.stride + iatom], toFixedForce(giz));
-      atomicAddFixed(&a.grad[3 * (size_t)a.stride + iatom], toFixedForce(giq));
+    // i sums over the four j lanes: every lane ends up with its own atom
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float lo = keepHalf(gi[0][q], gi[2][q], b4, 16), hi = keepHalf(gi[1][q], gi[3][q], b4, 16);
+      const float v = keepHalf(lo, hi, b3, 8);
+      if (v != 0.f)
+        atomicAddFixed(&a.grad[(size_t)q * a.stride + iatom], toFixedForce(q < 3 ? -v : v));
     }
+    __syncwarp();
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < d2; k += blockDim.x) {
-    if (s_gA[k] != 0.0f) atomicAdd(&a.gradAB[k], (double)s_gA[k]);
-    if (s_gB[k] != 0.0f) atomicAdd(&a.gradAB[d2 + k], (double)s_gB[k]);
+  for (int m = threadIdx.x; m < d2; m += blockDim.x) {
+    if (s_g[m].x != 0.0f) atomicAdd(&a.gradAB[m], (double)s_g[m].x);
+    if (s_g[m].y != 0.0f) atomicAdd(&a.gradAB[d2 + m], (double)s_g[m].y);
   }
 }
 
@@ -242,19 +310,38 @@ __global__ void adjointOutKernel(int n, const long long* __restrict__ g, int str
                          (float)(g[3 * (size_t)stride + i] * kForceScaleInv));
 }
 
-cudaError_t launchAdjoint(const AdjArgs& a, bool doSlow, int numSM, int n, float4* out,
-                          cudaStream_t st) {
-  const size_t shmem = (size_t)a.c.ljDim * a.c.ljDim * (sizeof(float2) + 2 * sizeof(float));
-  auto k = doSlow ? adjointKernel<true> : adjointKernel<false>;
-  if (shmem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
-    if (e != cudaSuccess) return e;
-  }
+template <bool S, bool SH>
+static cudaError_t launchAdj(const AdjArgs& a, size_t shmem, int numSM, cudaStream_t st) {
+  auto k = adjointKernel<S, SH>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
+  if (e != cudaSuccess) return e;
   int nb = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kAdjThreads, shmem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kAdjThreads, shmem);
   if (e != cudaSuccess) return e;
   k<<<numSM * (nb > 0 ? nb : 1), kAdjThreads, shmem, st>>>(a);
-  e = cudaGetLastError();
+  return cudaGetLastError();
+}
+
+cudaError_t launchAdjoint(const AdjArgs& args, bool doSlow, int numSM, int n, float4* out,
+                          cudaStream_t st) {
+  AdjArgs a = args;
+  const size_t tables = 2 * sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
+  // four interleaved copies of the slow table where they fit (fewer bank
+  // conflicts: neighbouring lanes read different copies), the table in global
+  // memory where not even one does
+  const size_t one = sizeof(float) * kAdjRow * (size_t)a.slowRows;
+  a.tabCopies = 4;
+  while (a.tabCopies > 1 && one * a.tabCopies > kAdjTableBytes) a.tabCopies /= 2;
+  cudaError_t e;
+  if (!doSlow) {
+    a.tabCopies = 1;
+    e = launchAdj<false, false>(a, tables, numSM, st);
+  } else if (one <= kAdjTableBytes) {
+    e = launchAdj<true, true>(a, tables + one * a.tabCopies, numSM, st);
+  } else {
+    a.tabCopies = 1;
+    e = launchAdj<true, false>(a, tables, numSM, st);
+  }
   if (e != cudaSuccess || !out) return e;
   adjointOutKernel<<<min((n + 255) / 256, numSM * 4), 256, 0, st>>>(n, a.grad, a.stride, out);
   return cudaGetLastError();

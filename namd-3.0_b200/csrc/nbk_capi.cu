@@ -977,6 +977,11 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
   a.latb = h->latb;
   a.latc = h->latc;
   a.c = h->c;
+  a.pk = h->pk;
+  a.slowTable = h->adjTable.p;
+  a.slowRows = h->slowTableRows;
+  a.slowStep = (float)h->slowStep;
+  a.slowInvStep = (float)(1.0 / h->slowStep);
   a.grad = h->adjGrad.p;
   a.stride = n;
   a.gradAB = d_gradAB;

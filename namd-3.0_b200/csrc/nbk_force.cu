@@ -342,16 +342,6 @@ __device__ __forceinline__ void reduceGroup(const int lane, LaneSums& L, long lo
   L = LaneSums{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 }
 
-// One reduction step over a pair of lanes (l and l ^ o): every lane keeps one
-// of its two values, the lane whose bit o is clear the first, the other the
-// second, and adds its partner's share of the one it keeps.
-__device__ __forceinline__ float keepHalf(const float first, const float second, const bool bit,
-                                          const int o) {
-  const float send = bit ? first : second;
-  const float keep = bit ? second : first;
-  return keep + __shfl_xor_sync(0xffffffffu, send, o);
-}
-
 // Block order: a 32 x 32 tile is 16 blocks of 8 i atoms by 8 j atoms. Lane
 // l = 8 lj + li (li = l & 7, lj = l >> 3) takes, of block (I, J), the pairs of
 // i = 8 I + li with j = 8 J + lj and j + 4 (elements x and y of the packed

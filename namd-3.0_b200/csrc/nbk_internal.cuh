@@ -346,6 +346,24 @@ __device__ __forceinline__ double warpSumD(double v) {
   return v;
 }
 
+// ---- what the tile-list kernels share ------------------------------------------
+// The next item of a work counter, drawn by lane 0 for the warp.
+__device__ __forceinline__ int drawItem(int* counter, const int lane) {
+  int W = 0;
+  if (lane == 0) W = atomicAdd(counter, 1);
+  return __shfl_sync(0xffffffffu, W, 0);
+}
+
+// One reduction step over a pair of lanes (l and l ^ o): every lane keeps one
+// of its two values, the lane whose bit o is clear the first, the other the
+// second, and adds its partner's share of the one it keeps.
+__device__ __forceinline__ float keepHalf(const float first, const float second, const bool bit,
+                                          const int o) {
+  const float send = bit ? first : second;
+  const float keep = bit ? second : first;
+  return keep + __shfl_xor_sync(0xffffffffu, send, o);
+}
+
 // ---- kernel argument blocks ---------------------------------------------------
 struct ForceArgs {
   const nbk_tile_list* lists;
