@@ -237,6 +237,17 @@ int tuneKey(const nbk_context* h, unsigned flags) {
          ((flags & NBK_SLOW) ? 1 : 0);
 }
 
+// Work items per tile list (log2) unless the tuner or the caller chose. A list
+// is one warp's work, about 3 us per tile. Resident warps: 16 per SM (2,368).
+// With fewer than about seven lists per warp the launch ends with most warps
+// idle behind the longest lists, so lists are split; splitting costs a list's
+// set-up per part, so large systems keep one part.
+int splitOf(const nbk_context* h, int key) {
+  if (h->tuneSplitLog2[key] >= 0) return h->tuneSplitLog2[key];
+  const int warps = 16 * h->numSM;
+  return h->numLists >= 7 * warps ? 0 : h->numLists >= 3 * warps ? 1 : 2;
+}
+
 // Force-kernel arguments for the handle's compacted lists, positions, lattice,
 // constants and replicas.
 ForceArgs refinedForceArgs(nbk_context* h, float cutoff2) {
@@ -354,7 +365,7 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   makePacked(h->c64, h->pk);
   for (int k = 0; k < 32; ++k) {
     h->tuneMinBlocks[k] = kDefaultMinBlocks;
-    h->tuneSplitLog2[k] = 0;
+    h->tuneSplitLog2[k] = -1;
     h->tuneMs[k] = 0.f;
   }
   // LJ tables (CudaNonbondedTables::buildVdwCoefTable, src/CudaNonbondedTables.C:110-148)
@@ -693,7 +704,7 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
   const bool shiftVirial = flags & NBK_VIRIAL;
   ForceArgs a = refinedForceArgs(h, cutoff2);
   const int key = tuneKey(h, flags);
-  a.splitLog2 = h->tuneSplitLog2[key];
+  a.splitLog2 = splitOf(h, key);
   NBK_CUDA(timedEvent(h, kTimedStart, st), "timing event");
   if (pairlist) {
     // refinement of the culled lists (the pairlist pass) and the order of
@@ -1272,11 +1283,13 @@ NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* str
     return setErr(NBK_ERR_CUDA, "nbk_autotune: event");
   }
   // shapes are timed back to back on a warm L2; another shape replaces the
-  // default (kDefaultMinBlocks CTAs per SM, one warp per list) only when it is
+  // default (kDefaultMinBlocks CTAs per SM, splitOf's warps per list) only when it is
   // at least 3% faster, so that timing noise does not pick a shape that loses
   // in use
   float bestMs = 1e30f, defaultMs = 1e30f;
-  int bestB = kDefaultMinBlocks, bestS = 0;
+  h->tuneSplitLog2[key] = -1;
+  const int defaultS = splitOf(h, key);
+  int bestB = kDefaultMinBlocks, bestS = defaultS;
   cudaError_t err = cudaSuccess;
   const int shapes[3] = {4, 5, 6};
   for (int bi = 0; bi < 3 && err == cudaSuccess; ++bi) {
@@ -1297,7 +1310,7 @@ NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* str
       if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e0, e1);
       if (err == cudaSuccess) {
         const float t = ms / iterations;
-        if (shapes[bi] == kDefaultMinBlocks && sl == 0) defaultMs = t;
+        if (shapes[bi] == kDefaultMinBlocks && sl == defaultS) defaultMs = t;
         if (t < bestMs) {
           bestMs = t;
           bestB = shapes[bi];
@@ -1311,7 +1324,7 @@ NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* str
   if (err != cudaSuccess) return setErr(NBK_ERR_CUDA, std::string("nbk_autotune: ") + cudaGetErrorString(err));
   if (!(bestMs < 0.97f * defaultMs)) {
     bestB = kDefaultMinBlocks;
-    bestS = 0;
+    bestS = defaultS;
     bestMs = defaultMs;
   }
   h->tuneMinBlocks[key] = bestB;
@@ -1326,7 +1339,7 @@ NBK_API int nbk_get_tuning(nbk_handle h, unsigned flags, int* minBlocksPerSM, in
   if (rc) return rc;
   const int key = tuneKey(h, flags & ~(unsigned)(NBK_PAIRLIST | NBK_CORRECTIONS));
   if (minBlocksPerSM) *minBlocksPerSM = h->tuneMinBlocks[key];
-  if (listSplit) *listSplit = 1 << h->tuneSplitLog2[key];
+  if (listSplit) *listSplit = 1 << splitOf(h, key);
   if (ms) *ms = h->tuneMs[key];
   return NBK_OK;
 }

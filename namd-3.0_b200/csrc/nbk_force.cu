@@ -31,10 +31,22 @@
 namespace nbk {
 
 constexpr int kForceWarps = 4;
-// Forces and the LJ energy are folded into fixed point once per group of
+// Forces and energies are folded into fixed point once per group of
 // kFoldTiles j tiles (groups counted from the start of the list; a list's
 // parts hold whole groups), so every sum is independent of the split.
 constexpr int kFoldTiles = 4;
+// The tiles [first, last] of part `part` of a list.
+__device__ __forceinline__ void listPart(const ForceArgs& a, const nbk_tile_list& tl, const int part,
+                                         int& first, int& last) {
+  const int split = 1 << a.splitLog2;
+  const int chunk = (((tl.jtileEnd - tl.jtileStart + split) >> a.splitLog2) + kFoldTiles - 1) &
+                    ~(kFoldTiles - 1);
+  first = tl.jtileStart + part * chunk;
+  last = min(tl.jtileEnd, first + chunk - 1);
+}
+__device__ __forceinline__ bool groupEnds(const nbk_tile_list& tl, const int jt, const int last) {
+  return ((jt - tl.jtileStart + 1) & (kFoldTiles - 1)) == 0 || jt == last;
+}
 constexpr int kForceThreads = kForceWarps * kWarp;
 constexpr size_t kForceTableBytes = 16 * 1024;  // slow force table copies per CTA
 
@@ -437,18 +449,13 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
   // draw short lists keep working instead of idling at the end
   const int split = 1 << a.splitLog2;
   for (;;) {
-    int W = 0;
-    if (lane == 0) W = atomicAdd(a.workCounter, 1);
-    W = __shfl_sync(0xffffffffu, W, 0);
+    const int W = drawItem(a.workCounter, lane);
     if (W >= numLists * split) break;
-    const int L = W >> a.splitLog2, part = W & (split - 1);
-    const nbk_tile_list tl = a.lists[L];
-    if (tl.jtileEnd < tl.jtileStart) continue;  // empty (warp-uniform)
-    const int chunk = ((((tl.jtileEnd - tl.jtileStart + split) >> a.splitLog2) + kFoldTiles - 1) /
-                       kFoldTiles) * kFoldTiles;
-    const int jtFirst = tl.jtileStart + part * chunk;
-    const int jtLast = min(tl.jtileEnd, jtFirst + chunk - 1);
-    if (jtLast < jtFirst) continue;  // this part has no tiles
+    const int part = W & (split - 1);
+    const nbk_tile_list tl = a.lists[W >> a.splitLog2];
+    int jtFirst, jtLast;
+    listPart(a, tl, part, jtFirst, jtLast);
+    if (jtLast < jtFirst) continue;  // this part has no tiles (warp-uniform)
     float3 la = a.lata, lb = a.latb, lc = a.latc;
     const char* ljRow = nullptr;  // batched: this replica's LJ table (global)
     if (doBatch) {
@@ -641,7 +648,7 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
       }
       if (doEnergy) s_evg[wib][lane] += (eV2.x + eV2.y) * (-1.0f / 6.0f);  // the terms are -6 E
       if (kLive) a.liveOut[(size_t)jt * kWarp + lane] = live;
-      if (((((jt - tl.jtileStart + 1) & (kFoldTiles - 1)) == 0) || jt == jtLast)) {
+      if (groupEnds(tl, jt, jtLast)) {
         // end of a tile group: its LJ energy and i forces into fixed point
         if (doEnergy) {
           s_ev[wib][lane] += toFixedEnergyF(s_evg[wib][lane]);
@@ -744,13 +751,15 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
   int npair = 0;       // interacting pairs counted by this lane (energy evaluations)
   LaneSums lsum{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   int curRep = 0;
+  const int split = 1 << a.splitLog2;
   for (;;) {
-    int L = 0;
-    if (lane == 0) L = atomicAdd(a.workCounter, 1);
-    L = __shfl_sync(0xffffffffu, L, 0);
-    if (L >= numLists) break;
-    const nbk_tile_list tl = a.lists[L];
-    if (tl.jtileEnd < tl.jtileStart) continue;  // empty (warp-uniform)
+    const int W = drawItem(a.workCounter, lane);
+    if (W >= numLists * split) break;
+    const int part = W & (split - 1);
+    const nbk_tile_list tl = a.lists[W >> a.splitLog2];
+    int jtFirst, jtLast;
+    listPart(a, tl, part, jtFirst, jtLast);
+    if (jtLast < jtFirst) continue;  // this part has no tiles (warp-uniform)
     float3 la = a.lata, lb = a.latb, lc = a.latc;
     if (doBatch) {
       const int rep = __ldg(&a.compRep[tl.icompute]);
@@ -778,17 +787,17 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
     int jsBlock = 0;
     unsigned liveNext = 0;
     float4 xjNext = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int jt = tl.jtileStart; jt <= tl.jtileEnd; ++jt) {
-      const int t = (jt - tl.jtileStart) & 31;
+    for (int jt = jtFirst; jt <= jtLast; ++jt) {
+      const int t = (jt - jtFirst) & 31;
       if (t == 0) {
         const int jtl = jt + lane;
-        jsBlock = jtl <= tl.jtileEnd ? a.tileJatomStart[jtl] : 0;
+        jsBlock = jtl <= jtLast ? a.tileJatomStart[jtl] : 0;
         liveNext = a.liveOut[(size_t)jt * kWarp + lane];
         xjNext = a.xyzq[__shfl_sync(0xffffffffu, jsBlock, 0) + lane];
       }
       const unsigned live = liveNext;
       const float4 xj = xjNext;
-      if (jt < tl.jtileEnd && t < 31) {
+      if (jt < jtLast && t < 31) {
         liveNext = a.liveOut[(size_t)(jt + 1) * kWarp + lane];
         xjNext = a.xyzq[__shfl_sync(0xffffffffu, jsBlock, t + 1) + lane];
       }
@@ -798,7 +807,7 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
         precisePass<doEnergy, doVirial, doSlow, kCopies>(live, lane, A, T, a.c,
                                                          lsum, npair);
       }
-      if (((jt - tl.jtileStart + 1) & (kFoldTiles - 1)) == 0 || jt == tl.jtileEnd)
+      if (groupEnds(tl, jt, jtLast))
         reduceGroup(lane, lsum, accQ);
     }
   }

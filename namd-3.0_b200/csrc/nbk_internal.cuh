@@ -392,7 +392,7 @@ struct ForceArgs {
   int stride;
   long long* acc;              // [kAccCount]
   int* workCounter;            // next work item to hand out (zeroed before the launch)
-  int splitLog2;               // force kernel: 2^splitLog2 work items per list
+  int splitLog2;               // force and precise kernel: 2^splitLog2 work items per list
   long long* compF;            // virial: [numComputes][6] i-force sums per compute (0..2 used)
   const double2* slowTable;    // [slowTableRows * kSlowTableRow / 2] phi_s rows (FP64)
   int slowTableRows;
