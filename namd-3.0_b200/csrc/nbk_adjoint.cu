@@ -37,29 +37,19 @@ __device__ __forceinline__ SlowRow slowRow(const float4 a, const float4 b, const
   return r;
 }
 
-// Adds (x, y) to a pair of sums in shared memory: one 64-bit compare-and-swap
-// for both, where two FP32 shared atomics would be two such loops.
-__device__ __forceinline__ void atomicAddPair(float2* p, const float x, const float y) {
-  unsigned long long* u = reinterpret_cast<unsigned long long*>(p);
-  unsigned long long old = *reinterpret_cast<volatile unsigned long long*>(u), seen;
-  do {
-    seen = old;
-    const float2 v = make_float2(__uint_as_float((unsigned)seen) + x,
-                                 __uint_as_float((unsigned)(seen >> 32)) + y);
-    old = atomicCAS(u, seen,
-                    (unsigned long long)__float_as_uint(v.x) |
-                        ((unsigned long long)__float_as_uint(v.y) << 32));
-  } while (old != seen);
-}
-
 // One warp per tile list, a tile as 16 blocks of 8 x 8 atoms as in the force
 // kernel (two j atoms per lane through packed FP32, i and j sums in registers
-// over a list and over a row of blocks). The kernel is bound by issue slots;
-// by diagonals of the tile, one pair per lane and step with the j sums rotated
-// between steps, it took 410 us at 24,000 atoms.
+// over a list part and over a row of blocks). By diagonals of the tile, one
+// pair per lane and step with the j sums rotated between steps, it took 410 us
+// at 24,000 atoms.
+//
+// The LJ gradients of a pair go to one of kAdjCopies FP64 tables in global
+// memory with two reductions that nothing waits for. In shared memory an FP32
+// add is a compare-and-swap loop, and the water model's few types make lanes
+// meet in it: with one loop for both sums the kernel took 313 us.
 template <bool doSlow, bool kShared>
 __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_constant__ AdjArgs a) {
-  // the slow table's copies (kShared), the LJ table (A, -B), the LJ gradients
+  // the slow table's copies (kShared), the LJ table (A, -B)
   extern __shared__ __align__(16) float4 s_dyn[];
   // i atoms: (-x, -x, -y, -y), (-z, -z, q, type), wF and wS as (x, x, y, y),
   // (Fz, Fz, Sz, Sz), (Sx, Sx, Sy, Sy)
@@ -73,13 +63,11 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
   const int dim = c.ljDim, d2 = dim * dim;
   const int tabEntries = kShared ? 2 * a.slowRows * a.tabCopies : 0;
   float2* s_lj = reinterpret_cast<float2*>(s_dyn + tabEntries);
-  float2* s_g = s_lj + d2;
+  double* const gAB = a.gradCopies + (size_t)(blockIdx.x % kAdjCopies) * 2 * d2;
   for (int m = threadIdx.x; m < tabEntries; m += blockDim.x)
     s_dyn[m] = a.slowTable[(unsigned)m / (unsigned)a.tabCopies];
-  for (int m = threadIdx.x; m < d2; m += blockDim.x) {
+  for (int m = threadIdx.x; m < d2; m += blockDim.x)
     s_lj[m] = make_float2(a.ljTable[m].x, -a.ljTable[m].y);
-    s_g[m] = make_float2(0.f, 0.f);
-  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int li = lane & 7, lj = lane >> 3;
@@ -91,9 +79,15 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
   const float sMax = a.slowStep * (float)(a.slowRows - 1);
   const int numLists = *a.numListsDev;
   for (;;) {
-    const int L = drawItem(a.workCounter, lane);
-    if (L >= numLists) break;
-    const nbk_tile_list tl = a.lists[L];
+    const int W = drawItem(a.workCounter, lane);
+    if (W >= numLists << a.splitLog2) break;
+    const nbk_tile_list tl = a.lists[W >> a.splitLog2];
+    // the part's tiles (contiguous parts of equal length, the last ones shorter)
+    const int split = 1 << a.splitLog2;
+    const int chunk = (tl.jtileEnd - tl.jtileStart + split) >> a.splitLog2;
+    const int jtFirst = tl.jtileStart + (W & (split - 1)) * chunk;
+    const int jtLast = min(tl.jtileEnd, jtFirst + chunk - 1);
+    if (jtLast < jtFirst) continue;  // warp-uniform
     const float3 sh = shiftOf(make_float3(tl.offsetXYZ.x, tl.offsetXYZ.y, tl.offsetXYZ.z), a.lata,
                               a.latb, a.latc);
     const int iatom = tl.iatomStart + lane;
@@ -113,7 +107,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
     float gi[4][4];  // sums of v (= -dL/dx_i) and of q_j dL/dqq for the atoms 8 I + li
 #pragma unroll
     for (int I = 0; I < 4; ++I) gi[I][0] = gi[I][1] = gi[I][2] = gi[I][3] = 0.f;
-    for (int jt = tl.jtileStart; jt <= tl.jtileEnd; ++jt) {
+    for (int jt = jtFirst; jt <= jtLast; ++jt) {
       const unsigned mask = a.tileExcls[jt].excl[lane];  // block order
       const int jstart = a.tileJatomStart[jt];
       {
@@ -267,8 +261,14 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
           const int ti = __float_as_int(i1.w);
           const bool wA = aA && ((ti | __float_as_int(tj.x)) & 1),
                      wB = aB && ((ti | __float_as_int(tj.y)) & 1);
-          if (wA) atomicAddPair(s_g + (tA >> 3), LA.x, LB.x);
-          if (wB) atomicAddPair(s_g + (tB >> 3), LA.y, LB.y);
+          if (wA) {
+            atomicAdd(gAB + (tA >> 3), (double)LA.x);
+            atomicAdd(gAB + d2 + (tA >> 3), (double)LB.x);
+          }
+          if (wB) {
+            atomicAdd(gAB + (tB >> 3), (double)LA.y);
+            atomicAdd(gAB + d2 + (tB >> 3), (double)LB.y);
+          }
         }
         // the row's sums over the eight i lanes; lane bits 1 and 0 keep one of
         // the components x, y, z, q of the lane's j atom
@@ -294,11 +294,16 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
     }
     __syncwarp();
   }
-  __syncthreads();
-  for (int m = threadIdx.x; m < d2; m += blockDim.x) {
-    if (s_g[m].x != 0.0f) atomicAdd(&a.gradAB[m], (double)s_g[m].x);
-    if (s_g[m].y != 0.0f) atomicAdd(&a.gradAB[d2 + m], (double)s_g[m].y);
-  }
+}
+
+// The LJ gradient tables' sum, copy by copy.
+__global__ void adjointTableKernel(int n, const double* __restrict__ copies, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < kAdjCopies; ++k) s += copies[(size_t)k * n + i];
+  out[i] = s;
 }
 
 // Fixed-point gradients -> float4 (gx, gy, gz, gq) per slot.
@@ -325,7 +330,8 @@ static cudaError_t launchAdj(const AdjArgs& a, size_t shmem, int numSM, cudaStre
 cudaError_t launchAdjoint(const AdjArgs& args, bool doSlow, int numSM, int n, float4* out,
                           cudaStream_t st) {
   AdjArgs a = args;
-  const size_t tables = 2 * sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
+  const int d2 = a.c.ljDim * a.c.ljDim;
+  const size_t tables = sizeof(float2) * (size_t)d2;
   // four interleaved copies of the slow table where they fit (fewer bank
   // conflicts: neighbouring lanes read different copies), the table in global
   // memory where not even one does
@@ -342,6 +348,9 @@ cudaError_t launchAdjoint(const AdjArgs& args, bool doSlow, int numSM, int n, fl
     a.tabCopies = 1;
     e = launchAdj<true, false>(a, tables, numSM, st);
   }
+  if (e != cudaSuccess) return e;
+  adjointTableKernel<<<(2 * d2 + 127) / 128, 128, 0, st>>>(2 * d2, a.gradCopies, a.gradAB);
+  e = cudaGetLastError();
   if (e != cudaSuccess || !out) return e;
   adjointOutKernel<<<min((n + 255) / 256, numSM * 4), 256, 0, st>>>(n, a.grad, a.stride, out);
   return cudaGetLastError();

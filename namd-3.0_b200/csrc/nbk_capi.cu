@@ -160,6 +160,7 @@ struct nbk_context {
   // adjoint
   DBuf<long long> adjGrad;
   DBuf<int> typeMask;
+  DBuf<double> adjAB;  // kAdjCopies tables of LJ gradients
   int adjStride = 0;
   // launch shape of the force kernel per flag combination (tuneKey): CTAs per
   // SM and log2 of the work items per list; set by nbk_autotune
@@ -461,6 +462,7 @@ NBK_API int nbk_destroy(nbk_handle h) {
   h->excTuples.release();
   h->adjGrad.release();
   h->typeMask.release();
+  h->adjAB.release();
   h->compRep.release();
   h->slotRep.release();
   h->repLat.release();
@@ -968,7 +970,9 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
     h->adjStride = n;
   }
   NBK_CUDA(cudaMemsetAsync(h->adjGrad.p, 0, sizeof(long long) * 4 * (size_t)n, st), "nbk_adjoint");
-  NBK_CUDA(cudaMemsetAsync(d_gradAB, 0, sizeof(double) * 2 * (size_t)dim * dim, st), "nbk_adjoint");
+  const size_t tables = 2 * (size_t)dim * dim * kAdjCopies;
+  NBK_CUDA(h->adjAB.ensure(tables), "nbk_adjoint");
+  NBK_CUDA(cudaMemsetAsync(h->adjAB.p, 0, sizeof(double) * tables, st), "nbk_adjoint");
   NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int), st), "nbk_adjoint");
   AdjArgs a{};
   a.lists = h->refinedLists();
@@ -996,12 +1000,14 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
   a.grad = h->adjGrad.p;
   a.stride = n;
   a.gradAB = d_gradAB;
+  a.gradCopies = h->adjAB.p;
+  a.splitLog2 = splitOf(h, tuneKey(h, NBK_ENERGY | flags));
   a.workCounter = h->counters.p + 2;
   NBK_CUDA(timedEvent(h, kTimedStart, st), "timing event");
   NBK_CUDA(launchAdjoint(a, slow, h->numSM, n, reinterpret_cast<float4*>(d_gradXQ), st), "adjoint kernel");
   NBK_CUDA(timedEvent(h, kTimedMid, st), "timing event");
   NBK_CUDA(timedEvent(h, kTimedStop, st), "timing event");
-  h->launches += d_gradXQ ? 2 : 1;
+  h->launches += d_gradXQ ? 3 : 2;
   if (d_gradFixed)
     NBK_CUDA(cudaMemcpyAsync(d_gradFixed, h->adjGrad.p, sizeof(long long) * 4 * (size_t)n,
                              cudaMemcpyDeviceToDevice, st), "nbk_adjoint: fixed-point copy");

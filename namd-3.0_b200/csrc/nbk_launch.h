@@ -107,6 +107,7 @@ void* mappedHostPointer(void* p);
 cudaError_t launchEnergyVirial(const long long* acc, nbk_virial_energy* out, cudaStream_t st,
                                int numReplicas = 1);
 
+constexpr int kAdjCopies = 16;
 struct AdjArgs {
   const nbk_tile_list* lists;
   const int* numListsDev;
@@ -127,7 +128,9 @@ struct AdjArgs {
   float slowStep, slowInvStep;
   long long* grad;       // SoA [4][stride]: gx, gy, gz, gq (fixed point, force scale)
   int stride;
-  double* gradAB;        // [2][ljDim*ljDim] (FP64 atomics)
+  double* gradAB;        // [2][ljDim*ljDim]
+  double* gradCopies;    // [kAdjCopies][2][ljDim*ljDim], zeroed (FP64 atomics)
+  int splitLog2;         // 2^splitLog2 work items per list
   int* workCounter;
 };
 cudaError_t launchAdjoint(const AdjArgs& a, bool doSlow, int numSM, int n, float4* out,
