@@ -105,7 +105,11 @@ struct PairTerms {
 // (z, q) pairs, and the current j tile as it is stored (FP32 x, y, z, q, exact
 // in FP64). A pair reads two 16-byte entries of its i atom and one of its j
 // atom: the j reads span the 512 bytes of the row, half of what FP64 rows
-// would, and the four conversions to FP64 cost less than the second load.
+// would, and the four conversions to FP64 cost less than the second load. The
+// j row is turned: atom j lies at 8 (j & 3) + (j >> 2). Neighbouring lanes walk
+// the pairs of neighbouring owners l, whose i atoms differ in l & 7 and whose j
+// atoms share l >> 3 and differ in their bit's J and e, so that with both rows
+// the lanes of a quarter warp read from different bank groups.
 struct Atoms64 {
   double2 ixy[kWarp], izq[kWarp];
   float4 j[kWarp];
@@ -160,7 +164,9 @@ __device__ __forceinline__ void precisePair(const PairTerms& u, const SlowTable&
     const double magic = 6755399441055744.0;
     const double t = fma(s, T.invStep, magic);
     const unsigned k = min((unsigned)__double2loint(t), T.last);
-    const double wq = fma(-T.step, (double)k, s);
+    // the row number back from t (no conversion); where the clamp acts, s is no
+    // pair's and only the row has to exist
+    const double wq = fma(-T.step, t - magic, s);
     double cf[kSlowTableDeg1];
 #pragma unroll
     for (int n = 0; n < kSlowTableDeg1; n += 2) {
@@ -203,9 +209,10 @@ __device__ __forceinline__ void precisePair(const PairTerms& u, const SlowTable&
 // repeats its last one, a real interacting pair (so its distance is not 0).
 __device__ __forceinline__ void pairTerms(const Atoms64& A, const int l, const int t,
                                           const bool valid, PairTerms& u) {
-  const int i = ((t & 3) << 3) | (l & 7), j = ((t & 28) ^ (l & 4)) | (l >> 3);
+  const int i = ((t & 3) << 3) | (l & 7);
   const double2 ia = A.ixy[i], ib = A.izq[i];
-  const float4 jb = A.j[j];
+  // j = ((t & 28) ^ (l & 4)) | (l >> 3), at its place in the turned row
+  const float4 jb = A.j[(l & 24) | ((t >> 2) ^ ((l >> 2) & 1))];
   u.dx = (double)jb.x - ia.x;
   u.dy = (double)jb.y - ia.y;
   u.dz = (double)jb.z - ib.x;
@@ -388,9 +395,12 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
   // the slow force table (kTable; a.tabCopies interleaved copies), then the LJ
   // table [ljDim*ljDim] as (A, -B) (single system)
   extern __shared__ __align__(16) float4 s_tab[];
-  // the list's i atoms, shifted: (-x, -x, -y, -y), then (-z, -z, q, byte
-  // offset of the type's LJ row)
-  __shared__ float4 s_i[kForceWarps][2][kWarp];
+  // the list's i atoms, shifted: (-x, -y, -z, q), and the byte offset of the
+  // type's LJ row. A 16-byte load takes four passes of the shared-memory pipe
+  // whatever the lanes share, so the coordinates are not kept twice for the
+  // packed instructions.
+  __shared__ float4 s_i[kForceWarps][kWarp];
+  __shared__ int s_it[kForceWarps][kWarp];
   // the j tile by pairs (j, j + 4) of a row's lanes: entry 4 J + lj holds
   // (x, x', y, y'), (z, z', q, q') and (type, type') as byte offsets in an LJ
   // row; the second copy, for the lanes with bit 2 set, holds j + 4 first
@@ -412,7 +422,8 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
   const int wib = threadIdx.x >> 5;
   const int li = lane & 7, lj = lane >> 3;
   const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4, b3 = lane & 8, b4 = lane & 16;
-  const unsigned adrI = sharedAddr(&s_i[wib][0][li]), adrJ = sharedAddr(&s_j[wib][b2][0][lj]),
+  const unsigned adrI = sharedAddr(&s_i[wib][li]), adrIT = sharedAddr(&s_it[wib][li]),
+                 adrJ = sharedAddr(&s_j[wib][b2][0][lj]),
                  adrT = sharedAddr(&s_jt[wib][b2][lj]);
   const NbkConst& c = a.c;
   const int dim = c.ljDim;
@@ -480,10 +491,9 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
     const int iatom = tl.iatomStart + lane;
     {
       const float4 xi = a.xyzq[iatom];
-      const float x = -__fadd_rn(xi.x, sh.x), y = -__fadd_rn(xi.y, sh.y),
-                  z = -__fadd_rn(xi.z, sh.z);
-      s_i[wib][0][lane] = make_float4(x, x, y, y);
-      s_i[wib][1][lane] = make_float4(z, z, xi.w, __int_as_float(a.vdwTypes[iatom] * dim * 8));
+      s_i[wib][lane] = make_float4(-__fadd_rn(xi.x, sh.x), -__fadd_rn(xi.y, sh.y),
+                                   -__fadd_rn(xi.z, sh.z), xi.w);
+      s_it[wib][lane] = a.vdwTypes[iatom] * dim * 8;
     }
 
     // this tile group's partial sums of the lane's four i atoms (8 I + li)
@@ -560,20 +570,20 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
 #pragma unroll
         for (int I = 0; I < 4; ++I) {
           if (!(rowAny & (0x11u << I))) continue;  // warp-uniform
-          const float4 ia = ldShared4(adrI + 128 * I), ib = ldShared4(adrI + 512 + 128 * I);
-          const float2 DX = add2(X, make_float2(ia.x, ia.y)),
-                       DY = add2(Y, make_float2(ia.z, ia.w)),
-                       DZ = add2(Z, make_float2(ib.x, ib.y));
+          const float4 xi = ldShared4(adrI + 128 * I);
+          const float2 DX = make_float2(X.x + xi.x, X.y + xi.x),
+                       DY = make_float2(Y.x + xi.y, Y.y + xi.y),
+                       DZ = make_float2(Z.x + xi.z, Z.y + xi.z);
           const float2 R2 = fma2(DZ, DZ, fma2(DX, DX, mul2(DY, DY)));  // dist2's order
           const bool aA = (mrow & (1u << I)) && (R2.x < c.cutoff2);
           const bool aB = (mrow & (0x10u << I)) && (R2.y < c.cutoff2);
           if (!__any_sync(0xffffffffu, aA || aB)) continue;
           if (kLive) liveRow |= (aA ? 1u << I : 0u) | (aB ? 0x10u << I : 0u);
-          const int ti = __float_as_int(ib.w);
+          const int ti = ldShared1(adrIT + 32 * I);
           const int tA = ti + __float_as_int(tj.x), tB = ti + __float_as_int(tj.y);
           const float2 abA = doBatch ? __ldg((const float2*)(ljRow + tA)) : ldShared2(adrLJ + tA);
           const float2 abB = doBatch ? __ldg((const float2*)(ljRow + tB)) : ldShared2(adrLJ + tB);
-          const float2 QQ = make_float2(ib.z * jb.z, ib.z * jb.w);
+          const float2 QQ = make_float2(xi.w * jb.z, xi.w * jb.w);
           float2 F, FS, E;
           pairForce2<doEnergy, doSlow, kTable>(R2, QQ, make_float2(abA.x, abB.x),
                                        make_float2(abA.y, abB.y), a.pk, T, F, FS, E);
@@ -803,7 +813,7 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
       }
       if (__any_sync(0xffffffffu, live != 0u)) {
         // the i rows and this j tile are visible after the pass's first __syncwarp
-        A.j[lane] = xj;
+        A.j[8 * (lane & 3) + (lane >> 2)] = xj;
         precisePass<doEnergy, doVirial, doSlow, kCopies>(live, lane, A, T, a.c,
                                                          lsum, npair);
       }
