@@ -692,12 +692,14 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     h->compFComputes = h->numComputes;
   }
   h->compF = h->force.p + 6 * (size_t)n;
-  NBK_CUDA(cudaMemsetAsync(h->force.p, 0,
-                           sizeof(long long) * 6 * ((size_t)n + (size_t)h->numComputes), st),
-           "nbk_nonbonded_force");
+  // the sums and the force, refinement and precise work counters; on a pairlist
+  // evaluation also the counts of lists and tiles, which the refinement makes
   const int accBlocks = h->nrep > 0 ? h->nrep : 1;
-  NBK_CUDA(cudaMemsetAsync(h->acc.p, 0, sizeof(long long) * kAccCount * (size_t)accBlocks, st),
-           "nbk_nonbonded_force");
+  NBK_CUDA(launchClear(h->force.p, 6 * ((size_t)n + (size_t)h->numComputes), h->acc.p,
+                       kAccCount * (size_t)accBlocks, h->counters.p + (pairlist ? 0 : 2),
+                       pairlist ? 5 : 3, h->numSM, st),
+           "nbk_nonbonded_force: clear");
+  h->launches += 1;
   h->lata = f3(lata);
   h->latb = f3(latb);
   h->latc = f3(latc);
@@ -736,8 +738,6 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     r.counts = h->counters.p;
     r.patchPairs = h->patchPairs.p;
     r.workCounter = h->counters.p + 3;
-    // lists and tiles kept; with them the work counters of all three kernels
-    NBK_CUDA(cudaMemsetAsync(h->counters.p, 0, sizeof(int) * 5, st), "nbk_nonbonded_force");
     NBK_CUDA(launchRefine(r, h->numSM, st), "pairlist refinement");
     if (h->listsSorted) {
       NBK_CUDA(launchSortLists(h->numLists, h->lists1.p, h->listActive.p, h->maxListLen,
@@ -755,8 +755,6 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
   a.lists = h->refinedLists();
   a.tileJatomStart = h->jatom2.p;
   a.tileExcls = h->excl2.p;
-  if (!pairlist)
-    NBK_CUDA(cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int) * 3, st), "nbk_nonbonded_force");
   if (needsPrecise(flags)) {
     NBK_CUDA(h->live.ensure((size_t)std::max(h->jcap, 1) * 32), "nbk_nonbonded_force");
     a.liveOut = h->live.p;
@@ -807,7 +805,7 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
       ca.repLat = h->repLat.p;
       ca.repLJExcl = h->repLJExcl.p;
     }
-    NBK_CUDA(launchCorrections(ca, flags, fs), "exclusion corrections");
+    NBK_CUDA(launchCorrections(ca, flags, !fork, fs), "exclusion corrections");
     h->launches += 1;
   }
   ShiftVirialArgs sv{};

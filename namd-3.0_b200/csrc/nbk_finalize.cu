@@ -1,9 +1,29 @@
 // Excluded / modified pair corrections, the fixed-point -> float4 force
 // output with the per-atom part of the virial, and the energy/virial read-out.
+#include <algorithm>
+
 #include "nbk_internal.cuh"
 #include "nbk_launch.h"
 
 namespace nbk {
+
+__global__ void clearKernel(ulonglong2* __restrict__ a, size_t na2, long long* __restrict__ b,
+                            size_t nb, int* __restrict__ c, int nc) {
+  admitSuccessor();
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (size_t k = i; k < na2; k += (size_t)gridDim.x * blockDim.x) a[k] = make_ulonglong2(0, 0);
+  for (size_t k = i; k < nb; k += (size_t)gridDim.x * blockDim.x) b[k] = 0;
+  for (size_t k = i; k < (size_t)nc; k += (size_t)gridDim.x * blockDim.x) c[k] = 0;
+}
+
+// a is 16-byte aligned (an allocation's start) and na even.
+cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int numSM,
+                        cudaStream_t st) {
+  const size_t most = std::max(na / 2, nb);
+  const int blocks = (int)std::min<size_t>((most + 255) / 256 + 1, 4 * (size_t)numSM);
+  clearKernel<<<blocks, 256, 0, st>>>(reinterpret_cast<ulonglong2*>(a), na / 2, b, nb, c, nc);
+  return cudaGetLastError();
+}
 
 // One thread per correction tuple (ComputeBondedCUDAKernel modifiedExclusionForce,
 // src/ComputeBondedCUDAKernel.cu:315-626, and exclusionForce, :632-778),
@@ -203,9 +223,13 @@ __global__ void correctionsKernel(const CorrArgs a) {
     }
   }
   if (doEnergy || doVirial) flushThreadAcc(a.acc, a.slotRep ? curRep : 0, acc);
+  // The forces are sums of integers, so this kernel may run beside the force
+  // kernel before it (both need only the cleared buffers); what comes after
+  // needs both.
+  waitForPredecessor();
 }
 
-cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, cudaStream_t st) {
+cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, bool besideForce, cudaStream_t st) {
   const bool E = flags & NBK_ENERGY, V = flags & NBK_VIRIAL, S = flags & NBK_SLOW;
   const int total = a.numModified + (S ? a.numExcluded : 0);
   if (total <= 0) return cudaSuccess;
@@ -215,8 +239,9 @@ cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, cudaStream_t st
   switch (idx) {
 #define NBK_CASE(i, e, v, s) \
   case i:                    \
+    if (besideForce) return launchOverlapped(correctionsKernel<e, v, s>, blocks, threads, 0, st, a); \
     correctionsKernel<e, v, s><<<blocks, threads, 0, st>>>(a); \
-    break;
+    return cudaGetLastError();
     NBK_CASE(0, false, false, false)
     NBK_CASE(1, false, false, true)
     NBK_CASE(2, false, true, false)
@@ -227,7 +252,7 @@ cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, cudaStream_t st
     NBK_CASE(7, true, true, true)
 #undef NBK_CASE
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 // Fixed point -> float4 forces (transposeForcesKernel's role,
@@ -246,6 +271,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
                    float4* __restrict__ outSH, int doSlow, int doVirial,
                    long long* __restrict__ accBase, const int* __restrict__ slotRep,
                    const ShiftVirialArgs shift) {
+  waitForPredecessor();
   long long v[9] = {};
   const int lane = threadIdx.x & 31;
   const int warpsTotal = (gridDim.x * blockDim.x) >> 5;
@@ -374,10 +400,8 @@ cudaError_t launchFinalizeForces(int n, const long long* force, int stride, cons
   const int blocks = min((n + threads - 1) / threads, 2 * numSM);
   ShiftVirialArgs sv{};
   if (shift && V) sv = *shift;
-  finalizeKernel<<<blocks, threads, 0, st>>>(n, force, stride, xyzq, outF, outS, outFHost,
-                                             outSHost, (flags & NBK_SLOW) ? 1 : 0, V ? 1 : 0, acc,
-                                             slotRep, sv);
-  return cudaGetLastError();
+  return launchOverlapped(finalizeKernel, blocks, threads, 0, st, n, force, stride, xyzq, outF, outS,
+                          outFHost, outSHost, (flags & NBK_SLOW) ? 1 : 0, V ? 1 : 0, acc, slotRep, sv);
 }
 
 void* mappedHostPointer(void* p) {

@@ -445,6 +445,10 @@ __global__ void __launch_bounds__(kForceThreads, MINB)
       s_lj[k] = make_float2(a.ljTable[k].x, -a.ljTable[k].y);
   }
   if (kTable || !doBatch) __syncthreads();
+  // the tables above belong to the handle; what follows needs the cleared
+  // buffers and the lists
+  waitForPredecessor();
+  admitSuccessor();
 
   const int numLists = a.numListsDev ? *a.numListsDev : a.numListsHost;
 
@@ -756,6 +760,7 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
     }
     __syncthreads();
   }
+  waitForPredecessor();
   const int numLists = a.numListsDev ? *a.numListsDev : a.numListsHost;
   long long accQ = 0;  // lane q < kNumQ: quantity q
   int npair = 0;       // interacting pairs counted by this lane (energy evaluations)
@@ -859,8 +864,7 @@ static cudaError_t launchPersistent(K kernel, OccCache& cache, int threads, size
     }
     blocks = cache.blocks[dev];
   }
-  kernel<<<numSM * blocks, threads, shmem, st>>>(a);
-  return cudaGetLastError();
+  return launchOverlapped(kernel, numSM * blocks, threads, shmem, st, a);
 }
 
 template <bool E, bool V, bool S, bool B, int MINB>

@@ -151,6 +151,14 @@ __device__ __forceinline__ float2 ldShared2(const unsigned a) {
   return v;
 }
 
+// Programmatic dependent launch: waits until the kernel before this one in the
+// stream has finished (nothing to wait for in an ordinary launch), and lets the
+// kernel after this one be scheduled before this one has finished.
+__device__ __forceinline__ void waitForPredecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void admitSuccessor() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // PTX approximate reciprocal, base-2 exponential and reciprocal square root
 // (rcp/ex2/rsqrt.approx.ftz.f32). The inputs here are normal numbers (r^2 is
 // at least the square of the shortest pair distance, 2^(gaussK r^2) lies in

@@ -10,6 +10,30 @@
 
 namespace nbk {
 
+// Launches a kernel that may be scheduled while the kernel before it in the
+// stream still runs; it calls waitForPredecessor before it uses anything that
+// one writes. Saves the gap between two small kernels.
+template <typename... P, typename... A>
+cudaError_t launchOverlapped(void (*kernel)(P...), int blocks, int threads, size_t shmem,
+                             cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = shmem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Zeroes the 64-bit words a[0, na), b[0, nb) and the 32-bit words c[0, nc) in
+// one launch (three memsets cost three gaps).
+cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int numSM,
+                        cudaStream_t st);
+
 // Pair-math constants from the caller's parameters (nbk_consts.cu); shared by
 // the handle and by the allocation-free entry point.
 void makeConstants(const nbk_params& p, int ljDim, NbkConst& c, NbkConst64& k);
@@ -77,7 +101,9 @@ struct CorrArgs {
   const float3* repLat;        // [3*numReplicas]
   const float2* repLJExcl;     // [numReplicas][ljDim*ljDim] (A14 - A, B14 - B) * scaling
 };
-cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, cudaStream_t st);
+// besideForce: the kernel before it in the stream is the force kernel, whose end
+// it does not need (its own end waits for it).
+cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, bool besideForce, cudaStream_t st);
 
 // The lattice-shift part of the virial, (sum_i F_i) (x) shift per compute,
 // from the exact integer i-force sums the force kernel leaves per compute.

@@ -154,7 +154,7 @@ extern "C" NBK_API int nbk_exclusion_force_noalloc(
   ca.acc = acc;
   int numSM = 148;
   cudaDeviceGetAttribute(&numSM, cudaDevAttrMultiProcessorCount, device);
-  e = launchCorrections(ca, flags, st);
+  e = launchCorrections(ca, flags, false, st);
   if (e == cudaSuccess)
     e = launchFinalizeForces(n, force, n, ca.xyzq, reinterpret_cast<float4*>(d_forces),
                              (flags & NBK_SLOW) ? reinterpret_cast<float4*>(d_forcesSlow) : nullptr,
