@@ -692,12 +692,17 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     h->compFComputes = h->numComputes;
   }
   h->compF = h->force.p + 6 * (size_t)n;
+  int lengths = 0;  // words of the histogram of list lengths
+  if (pairlist && h->nrep == 0) {
+    lengths = h->maxListLen + 1;
+    NBK_CUDA(h->lenHist.ensure(lengths), "nbk_nonbonded_force");
+  }
   // the sums and the force, refinement and precise work counters; on a pairlist
   // evaluation also the counts of lists and tiles, which the refinement makes
   const int accBlocks = h->nrep > 0 ? h->nrep : 1;
   NBK_CUDA(launchClear(h->force.p, 6 * ((size_t)n + (size_t)h->numComputes), h->acc.p,
                        kAccCount * (size_t)accBlocks, h->counters.p + (pairlist ? 0 : 2),
-                       pairlist ? 5 : 3, h->numSM, st),
+                       pairlist ? 5 : 3, h->lenHist.p, lengths, h->numSM, st),
            "nbk_nonbonded_force: clear");
   h->launches += 1;
   h->lata = f3(lata);
@@ -717,9 +722,6 @@ NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flag
     h->listsSorted = h->nrep == 0;
     if (h->listsSorted) {
       NBK_CUDA(h->lists2.ensure(nl), "nbk_nonbonded_force");
-      NBK_CUDA(h->lenHist.ensure((size_t)h->maxListLen + 1), "nbk_nonbonded_force");
-      NBK_CUDA(cudaMemsetAsync(h->lenHist.p, 0, sizeof(int) * ((size_t)h->maxListLen + 1), st),
-               "nbk_nonbonded_force");
     } else {
       NBK_CUDA(h->listsCompact.ensure(nl), "nbk_nonbonded_force");
     }

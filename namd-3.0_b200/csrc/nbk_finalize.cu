@@ -8,20 +8,22 @@
 namespace nbk {
 
 __global__ void clearKernel(ulonglong2* __restrict__ a, size_t na2, long long* __restrict__ b,
-                            size_t nb, int* __restrict__ c, int nc) {
+                            size_t nb, int* __restrict__ c, int nc, int* __restrict__ d, int nd) {
   admitSuccessor();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   for (size_t k = i; k < na2; k += (size_t)gridDim.x * blockDim.x) a[k] = make_ulonglong2(0, 0);
   for (size_t k = i; k < nb; k += (size_t)gridDim.x * blockDim.x) b[k] = 0;
   for (size_t k = i; k < (size_t)nc; k += (size_t)gridDim.x * blockDim.x) c[k] = 0;
+  for (size_t k = i; k < (size_t)nd; k += (size_t)gridDim.x * blockDim.x) d[k] = 0;
 }
 
 // a is 16-byte aligned (an allocation's start) and na even.
-cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int numSM,
-                        cudaStream_t st) {
+cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int* d,
+                        int nd, int numSM, cudaStream_t st) {
   const size_t most = std::max(na / 2, nb);
   const int blocks = (int)std::min<size_t>((most + 255) / 256 + 1, 4 * (size_t)numSM);
-  clearKernel<<<blocks, 256, 0, st>>>(reinterpret_cast<ulonglong2*>(a), na / 2, b, nb, c, nc);
+  clearKernel<<<blocks, 256, 0, st>>>(reinterpret_cast<ulonglong2*>(a), na / 2, b, nb, c, nc,
+                                       d, nd);
   return cudaGetLastError();
 }
 

@@ -29,10 +29,10 @@ cudaError_t launchOverlapped(void (*kernel)(P...), int blocks, int threads, size
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// Zeroes the 64-bit words a[0, na), b[0, nb) and the 32-bit words c[0, nc) in
-// one launch (three memsets cost three gaps).
-cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int numSM,
-                        cudaStream_t st);
+// Zeroes the 64-bit words a[0, na), b[0, nb) and the 32-bit words c[0, nc),
+// d[0, nd) in one launch (memsets cost a gap each).
+cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int* d,
+                        int nd, int numSM, cudaStream_t st);
 
 // Pair-math constants from the caller's parameters (nbk_consts.cu); shared by
 // the handle and by the allocation-free entry point.

@@ -18,6 +18,7 @@ namespace nbk {
 // One warp per 32-atom tile: min/max reduction over the tile's atoms
 // (buildBoundingBoxesKernel, src/CudaTileListKernel.cu:242-281).
 __global__ void bboxKernel(int numTiles, const float4* __restrict__ xyzq, BBox* __restrict__ bb) {
+  admitSuccessor();
   const int lane = threadIdx.x & 31;
   const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < numTiles; t += warpsPerGrid) {
@@ -53,8 +54,10 @@ __device__ __forceinline__ float bbDist2(const BBox& a, const BBox& b) {
   return dx * dx + dy * dy + dz * dz;
 }
 
-// One warp per (compute, i-tile): j tiles of the partner patch whose box is
-// within the pairlist cutoff (self computes: j-tile >= i-tile).
+// Half a warp per (compute, i-tile): j tiles of the partner patch whose box is
+// within the pairlist cutoff (self computes: j-tile >= i-tile). The kernel is a
+// chain of three dependent loads per list; most patches have at most 16 tiles,
+// so that a whole warp per list left half of it idle and took twice the waves.
 __global__ void buildListsKernel(int numLists, const ListSeed* __restrict__ seeds,
                                  const nbk_compute_record* __restrict__ computes,
                                  const nbk_patch_record* __restrict__ patches,
@@ -62,9 +65,11 @@ __global__ void buildListsKernel(int numLists, const ListSeed* __restrict__ seed
                                  const int* __restrict__ compRep, const float3* __restrict__ repLat,
                                  float cull2, nbk_tile_list* __restrict__ lists,
                                  PatchPair* __restrict__ pp, int* __restrict__ tileJatomStart) {
-  const int lane = threadIdx.x & 31;
-  const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-  for (int L = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; L < numLists; L += warpsPerGrid) {
+  waitForPredecessor();
+  const int lane = threadIdx.x & 15;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  const int halvesPerGrid = (gridDim.x * blockDim.x) >> 4;
+  for (int L = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; L < numLists; L += halvesPerGrid) {
     const ListSeed sd = seeds[L];
     const nbk_compute_record cr = computes[sd.icompute];
     const nbk_patch_record p1 = patches[cr.patchInd.x];
@@ -85,11 +90,11 @@ __global__ void buildListsKernel(int numLists, const ListSeed* __restrict__ seed
     bi.z += sh.z;
     const int ntiles2 = (p2.numAtoms + 31) / 32;
     int count = 0;
-    for (int k0 = 0; k0 < ntiles2; k0 += 32) {
+    for (int k0 = 0; k0 < ntiles2; k0 += 16) {  // the same for the half warp
       const int k = k0 + lane;
       bool pass = false;
       if (k < ntiles2 && (!self || k >= sd.itile)) pass = bbDist2(bi, bb[p2.atomStart / 32 + k]) < cull2;
-      const unsigned ball = __ballot_sync(0xffffffffu, pass);
+      const unsigned ball = __ballot_sync(half, pass) >> (threadIdx.x & 16);
       if (pass) {
         const int rank = __popc(ball & ((1u << lane) - 1u));
         tileJatomStart[sd.jcapStart + count + rank] = p2.atomStart + k * 32;
@@ -193,6 +198,8 @@ __global__ void __launch_bounds__(128) refineKernel(const __grid_constant__ Forc
   const float2 nPlc2 = f2(-a.c.plcutoff2);
   float* const p0 = reinterpret_cast<float*>(&s_p0[wib][lane & 15]) + (lane >> 4);
   float* const p1 = reinterpret_cast<float*>(&s_p1[wib][lane & 15]) + (lane >> 4);
+  waitForPredecessor();
+  admitSuccessor();
   int nexcl = 0, curRep = 0, tiles = 0;
   for (;;) {
     int L = 0;
@@ -332,8 +339,7 @@ cudaError_t launchRefine(const ForceArgs& a, int numSM, cudaStream_t st) {
     blocks = nb > 0 ? nb : 1;
     cachedBlocks.store(blocks, std::memory_order_relaxed);
   }
-  refineKernel<<<numSM * blocks, 128, 0, st>>>(a);
-  return cudaGetLastError();
+  return launchOverlapped(refineKernel, numSM * blocks, 128, 0, st, a);
 }
 
 // The refined lists in order of decreasing length (the order sortTileLists
@@ -348,6 +354,8 @@ cudaError_t launchRefine(const ForceArgs& a, int numSM, cudaStream_t st) {
 // Descending offsets of the lengths 1..maxLen and the number of lists, by one
 // warp from the histogram that the refinement counted.
 __global__ void listLengthScanKernel(int maxLen, int* __restrict__ hist, int* __restrict__ counts) {
+  waitForPredecessor();
+  admitSuccessor();
   const int lane = threadIdx.x;
   int off = 0;
   for (int top = maxLen; top >= 1; top -= 32) {
@@ -368,6 +376,8 @@ __global__ void listLengthScanKernel(int maxLen, int* __restrict__ hist, int* __
 __global__ void listScatterKernel(int n, const nbk_tile_list* __restrict__ src,
                                   const int* __restrict__ listActive, int maxLen,
                                   int* __restrict__ cursor, nbk_tile_list* __restrict__ dst) {
+  waitForPredecessor();
+  admitSuccessor();
   const int lane = threadIdx.x & 31;
   for (int L0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; L0 < n; L0 += gridDim.x * blockDim.x) {
     const int L = L0 + lane;
@@ -391,9 +401,10 @@ cudaError_t launchSortLists(int numLists, const nbk_tile_list* src, const int* l
                             cudaStream_t st) {
   if (numLists <= 0) return cudaSuccess;
   const int blocks = min((numLists + 255) / 256, numSM * 4);
-  listLengthScanKernel<<<1, 32, 0, st>>>(maxLen, hist, counts);
-  listScatterKernel<<<blocks, 256, 0, st>>>(numLists, src, listActive, maxLen, hist, dst);
-  return cudaGetLastError();
+  const cudaError_t e = launchOverlapped(listLengthScanKernel, 1, 32, 0, st, maxLen, hist, counts);
+  if (e != cudaSuccess) return e;
+  return launchOverlapped(listScatterKernel, blocks, 256, 0, st, numLists, src, listActive, maxLen,
+                          hist, dst);
 }
 
 // Export: list k's tiles from its own slots to the place in packed arrays that
@@ -440,11 +451,9 @@ cudaError_t launchBuildLists(int numLists, const ListSeed* seeds,
                              cudaStream_t st) {
   if (numLists <= 0) return cudaSuccess;
   const int threads = 256;
-  const int blocks = min((numLists + 7) / 8, 8192);
-  buildListsKernel<<<blocks, threads, 0, st>>>(numLists, seeds, computes, patches, bb, lata, latb,
-                                               latc, compRep, repLat, cull2, lists, pp,
-                                               tileJatomStart);
-  return cudaGetLastError();
+  const int blocks = min((numLists + 15) / 16, 8192);
+  return launchOverlapped(buildListsKernel, blocks, threads, 0, st, numLists, seeds, computes, patches,
+                          bb, lata, latb, latc, compRep, repLat, cull2, lists, pp, tileJatomStart);
 }
 
 cudaError_t launchCompact(int numLists, const nbk_tile_list* src, const int* listActive,
