@@ -52,6 +52,8 @@ __device__ __forceinline__ void flushThreadAcc(long long* accBase, int rep, long
   }
 }
 
+constexpr int kCorrThreads = 256;
+
 // Forces are FP32 (fixed-point accumulated, like the nonbonded kernel's);
 // energies and the slow virial are formed per tuple in FP64 from FP64
 // geometry (the shift formed in FP64 from the FP32 offsets and lattice), the
@@ -224,7 +226,31 @@ __global__ void correctionsKernel(const CorrArgs a) {
       for (int p = 0; p < 9; ++p) acc[kAccVir + p] += toFixedEnergy(Fi[p / 3] * S[p % 3]);
     }
   }
-  if (doEnergy || doVirial) flushThreadAcc(a.acc, a.slotRep ? curRep : 0, acc);
+  if (doEnergy || doVirial) {
+    // A block whose threads all hold one replica's sums adds each word once:
+    // adds of every warp to the same 21 words took longer than the tuples.
+    __shared__ long long s_acc[kCorrThreads / 32][kAccCount - 3];
+    const int rep = a.slotRep ? curRep : 0;
+    __shared__ int s_rep;
+    if (threadIdx.x == 0) s_rep = rep;
+    __syncthreads();
+    const int rep0 = s_rep;
+    if (__syncthreads_and(rep == rep0)) {
+#pragma unroll
+      for (int p = 0; p < kAccCount - 3; ++p) {
+        const long long v = warpSumLL(acc[p]);
+        if (lane == 0) s_acc[threadIdx.x >> 5][p] = v;
+      }
+      __syncthreads();
+      if (threadIdx.x < kAccCount - 3) {
+        long long v = 0;
+        for (int w = 0; w < kCorrThreads / 32; ++w) v += s_acc[w][threadIdx.x];
+        if (v) atomicAddFixed(&a.acc[(size_t)rep0 * kAccCount + threadIdx.x], (unsigned long long)v);
+      }
+    } else {
+      flushThreadAcc(a.acc, rep, acc);
+    }
+  }
   // The forces are sums of integers, so this kernel may run beside the force
   // kernel before it (both need only the cleared buffers); what comes after
   // needs both.
@@ -235,7 +261,7 @@ cudaError_t launchCorrections(const CorrArgs& a, unsigned flags, bool besideForc
   const bool E = flags & NBK_ENERGY, V = flags & NBK_VIRIAL, S = flags & NBK_SLOW;
   const int total = a.numModified + (S ? a.numExcluded : 0);
   if (total <= 0) return cudaSuccess;
-  const int threads = 256;
+  const int threads = kCorrThreads;
   const int blocks = min((total + threads - 1) / threads, 2048);
   const int idx = (E ? 4 : 0) | (V ? 2 : 0) | (S ? 1 : 0);
   switch (idx) {
@@ -281,18 +307,26 @@ __global__ void __launch_bounds__(kFinalizeThreads)
   const int per = ((n + warpsTotal - 1) / warpsTotal + 31) & ~31;
   const int iEnd = min(n, (gw + 1) * per);
   int curRep = 0;
+  // the warp's sums into the replicas its threads accumulated for: one add per
+  // word where they hold one replica
+  auto flush = [&]() {
+    const int rep0 = __shfl_sync(0xffffffffu, curRep, 0);
+    const bool uniform = __all_sync(0xffffffffu, curRep == rep0);
+#pragma unroll
+    for (int p = 0; p < 9; ++p) {
+      const long long s = uniform ? warpSumLL(v[p]) : v[p];
+      if (s != 0 && (!uniform || lane == 0))
+        atomicAddFixed(&accBase[(size_t)curRep * kAccCount + kAccVir + p], (unsigned long long)s);
+      v[p] = 0;
+    }
+  };
   for (int i0 = gw * per; i0 < iEnd; i0 += 32) {
     const int i = i0 + lane;
     const bool valid = i < iEnd;
     if (doVirial && slotRep) {
       const int rep = valid ? slotRep[i] : curRep;
       if (__any_sync(0xffffffffu, rep != curRep)) {
-        // flush per thread into the replica it accumulated for
-#pragma unroll
-        for (int p = 0; p < 9; ++p) {
-          if (v[p] != 0) atomicAddFixed(&accBase[(size_t)curRep * kAccCount + kAccVir + p], (unsigned long long)v[p]);
-          v[p] = 0;
-        }
+        flush();
         curRep = rep;
       }
     }
@@ -327,17 +361,19 @@ __global__ void __launch_bounds__(kFinalizeThreads)
   // reduceNonbondedVirialKernel / reduceVirialEnergyKernel,
   // src/CudaComputeNonbondedKernel.cu:1649-1920). Each compute's product is
   // rounded once, so the result does not depend on how lists were scheduled.
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < shift.numComputes;
-       c += gridDim.x * blockDim.x) {
-    const int rep = shift.compRep ? shift.compRep[c] : 0;
-    if (rep != curRep) {
-#pragma unroll
-      for (int p = 0; p < 9; ++p) {
-        if (v[p] != 0) atomicAddFixed(&accBase[(size_t)curRep * kAccCount + kAccVir + p], (unsigned long long)v[p]);
-        v[p] = 0;
-      }
+  // A warp takes a contiguous range, like the slots (with the range of one
+  // thread spread over all replicas every thread flushed by itself: 60 us for
+  // 64 replicas of 836,215 atoms in all).
+  const int perC = ((shift.numComputes + warpsTotal - 1) / warpsTotal + 31) & ~31;
+  const int cEnd = min(shift.numComputes, (gw + 1) * perC);
+  for (int c0 = gw * perC; c0 < cEnd; c0 += 32) {
+    const int c = c0 + lane;
+    const int rep = c < cEnd && shift.compRep ? shift.compRep[c] : curRep;
+    if (__any_sync(0xffffffffu, rep != curRep)) {
+      flush();
       curRep = rep;
     }
+    if (c >= cEnd) continue;
     const long long* Fc = shift.compF + 6 * (size_t)c;
     const nbk_compute_record cr = shift.computes[c];
     float3 la = shift.lata, lb = shift.latb, lc = shift.latc;
@@ -397,9 +433,10 @@ cudaError_t launchFinalizeForces(int n, const long long* force, int stride, cons
   const bool V = flags & NBK_VIRIAL;
   if (!V && !outF && !outS && !outFHost && !outSHost) return cudaSuccess;
   const int threads = kFinalizeThreads;
-  // two blocks per SM keep enough loads in flight (one per SM left the
-  // kernel latency-bound: 11 -> 9 us at 97k slots)
-  const int blocks = min((n + threads - 1) / threads, 2 * numSM);
+  // two blocks per SM keep enough loads in flight for small systems (one per SM
+  // left the kernel latency-bound: 11 -> 9 us at 97k slots), six for large ones
+  // (36 -> 28 us at 1.1M slots)
+  const int blocks = min((n + threads - 1) / threads, (n >= 1024 * numSM ? 6 : 2) * numSM);
   ShiftVirialArgs sv{};
   if (shift && V) sv = *shift;
   return launchOverlapped(finalizeKernel, blocks, threads, 0, st, n, force, stride, xyzq, outF, outS,
