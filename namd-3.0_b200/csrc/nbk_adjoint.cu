@@ -51,9 +51,8 @@ template <bool doSlow, bool kShared>
 __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_constant__ AdjArgs a) {
   // the slow table's copies (kShared), the LJ table (A, -B)
   extern __shared__ __align__(16) float4 s_dyn[];
-  // i atoms: (-x, -x, -y, -y), (-z, -z, q, type), wF and wS as (x, x, y, y),
-  // (Fz, Fz, Sz, Sz), (Sx, Sx, Sy, Sy)
-  __shared__ float4 s_i[kAdjWarps][5][kWarp];
+  // i atoms: (-x, -y, -z, q), (wF, type), (wS, -)
+  __shared__ float4 s_i[kAdjWarps][3][kWarp];
   // j atoms by pairs (j, j + 4), two copies in turned order as in the force
   // kernel: (x, x', y, y'), (z, z', q, q'), -wF and -wS likewise; types
   __shared__ float4 s_j[kAdjWarps][2][5][16];
@@ -98,11 +97,9 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
       const int ty = a.vdwTypes[iatom];
       const float x = -__fadd_rn(xi.x, sh.x), y = -__fadd_rn(xi.y, sh.y), z = -__fadd_rn(xi.z, sh.z);
       const int off = ty * dim * 8 + (a.typeMask[ty] != 0 ? 1 : 0);
-      s_i[wib][0][lane] = make_float4(x, x, y, y);
-      s_i[wib][1][lane] = make_float4(z, z, xi.w, __int_as_float(off));
-      s_i[wib][2][lane] = make_float4(wf.x, wf.x, wf.y, wf.y);
-      s_i[wib][3][lane] = make_float4(wf.z, wf.z, ws.z, ws.z);
-      s_i[wib][4][lane] = make_float4(ws.x, ws.x, ws.y, ws.y);
+      s_i[wib][0][lane] = make_float4(x, y, z, xi.w);
+      s_i[wib][1][lane] = make_float4(wf.x, wf.y, wf.z, __int_as_float(off));
+      s_i[wib][2][lane] = ws;
     }
     float gi[4][4];  // sums of v (= -dL/dx_i) and of q_j dL/dqq for the atoms 8 I + li
 #pragma unroll
@@ -154,21 +151,21 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
         for (int I = 0; I < 4; ++I) {
           if (!(rowAny & (0x11u << I))) continue;  // warp-uniform
           const unsigned ai = adrI + 128 * I;
-          const float4 i0 = ldShared4(ai), i1 = ldShared4(ai + 512);
-          const float2 DX = add2(make_float2(j0.x, j0.y), make_float2(i0.x, i0.y)),
-                       DY = add2(make_float2(j0.z, j0.w), make_float2(i0.z, i0.w)),
-                       DZ = add2(make_float2(j1.x, j1.y), make_float2(i1.x, i1.y));
+          const float4 xi = ldShared4(ai);
+          const float2 DX = make_float2(j0.x + xi.x, j0.y + xi.x),
+                       DY = make_float2(j0.z + xi.y, j0.w + xi.y),
+                       DZ = make_float2(j1.x + xi.z, j1.y + xi.z);
           const float2 R2 = fma2(DZ, DZ, fma2(DX, DX, mul2(DY, DY)));  // dist2's order
           const bool aA = (mrow & (1u << I)) && (R2.x < c.cutoff2);
           const bool aB = (mrow & (0x10u << I)) && (R2.y < c.cutoff2);
           if (!__any_sync(0xffffffffu, aA || aB)) continue;
-          const float4 i2 = ldShared4(ai + 1024), i3 = ldShared4(ai + 1536);
-          const float2 UX = add2(make_float2(i2.x, i2.y), make_float2(j2.x, j2.y)),
-                       UY = add2(make_float2(i2.z, i2.w), make_float2(j2.z, j2.w)),
-                       UZ = add2(make_float2(i3.x, i3.y), make_float2(j3.x, j3.y));
+          const float4 wi = ldShared4(ai + 512);
+          const float2 UX = make_float2(wi.x + j2.x, wi.x + j2.y),
+                       UY = make_float2(wi.y + j2.z, wi.y + j2.w),
+                       UZ = make_float2(wi.z + j3.x, wi.z + j3.y);
           const float2 pF = fma2(UZ, DZ, fma2(UY, DY, mul2(UX, DX)));
-          const int tA = __float_as_int(i1.w) + __float_as_int(tj.x),
-                    tB = __float_as_int(i1.w) + __float_as_int(tj.y);
+          const int ti = __float_as_int(wi.w);
+          const int tA = ti + __float_as_int(tj.x), tB = ti + __float_as_int(tj.y);
           const float2 abA = ldShared2(adrLJ + (tA & ~7)), abB = ldShared2(adrLJ + (tB & ~7));
           const float2 A = make_float2(abA.x, abB.x), nB = make_float2(abA.y, abB.y);
           const float2 rinv = make_float2(rsqrtApprox(R2.x), rsqrtApprox(R2.y));
@@ -193,7 +190,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
           const float2 hA = mul2(s6, fma2(si, fma2(f2(42.0f), m, mul2(f2(-12.0f), S1)), S2));
           const float2 hB = mul2(s3, fma2(si, fma2(f2(12.0f), m, mul2(f2(-6.0f), S1)), S2));
           const float2 hlj = fma2(A, hA, mul2(nB, hB));  // g_lj' / 2
-          const float2 qi = f2(i1.z), qq = mul2(qi, QJ);
+          const float2 qi = f2(xi.w), qq = mul2(qi, QJ);
           const float2 gf = add2(k.rc3inv, neg2(rinv3));
           const float2 hf = mul2(f2(0.75f), mul2(rinv3, si));  // g_f' / 2
           const float2 phif = add2(rinv, neg2(fma2(f2(c.hB), R2, f2(c.hA))));
@@ -204,10 +201,10 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
           float2 dqq = fma2(pF, gf, mul2(f2(a.cE), phif));
           float2 VX = mul2(g, UX), VY = mul2(g, UY), VZ = mul2(g, UZ);
           if constexpr (doSlow) {
-            const float4 i4 = ldShared4(ai + 2048);
-            const float2 WX = add2(make_float2(i4.x, i4.y), make_float2(j4.x, j4.y)),
-                         WY = add2(make_float2(i4.z, i4.w), make_float2(j4.z, j4.w)),
-                         WZ = add2(make_float2(i3.z, i3.w), make_float2(j3.z, j3.w));
+            const float4 vi = ldShared4(ai + 1024);
+            const float2 WX = make_float2(vi.x + j4.x, vi.x + j4.y),
+                         WY = make_float2(vi.y + j4.z, vi.y + j4.w),
+                         WZ = make_float2(vi.z + j3.z, vi.z + j3.w);
             const float2 pS = fma2(WZ, DZ, fma2(WY, DY, mul2(WX, DX)));
             const float2 sc = make_float2(fminf(R2.x, sMax), fminf(R2.y, sMax));
             const float2 t = fma2(sc, f2(a.slowInvStep), f2(kRowMagic));
@@ -258,7 +255,6 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
           // dL/dA = pF gA + cV s^-6 S, dL/dB = -(pF gnB + cV s^-3 S)
           const float2 cS6 = mul2(f2(a.cV), S);
           const float2 LA = fma2(pF, gA, mul2(cS6, s6)), LB = neg2(fma2(pF, gnB, mul2(cS6, s3)));
-          const int ti = __float_as_int(i1.w);
           const bool wA = aA && ((ti | __float_as_int(tj.x)) & 1),
                      wB = aB && ((ti | __float_as_int(tj.y)) & 1);
           if (wA) {
@@ -332,11 +328,11 @@ cudaError_t launchAdjoint(const AdjArgs& args, bool doSlow, int numSM, int n, fl
   AdjArgs a = args;
   const int d2 = a.c.ljDim * a.c.ljDim;
   const size_t tables = sizeof(float2) * (size_t)d2;
-  // four interleaved copies of the slow table where they fit (fewer bank
-  // conflicts: neighbouring lanes read different copies), the table in global
-  // memory where not even one does
+  // eight interleaved copies of the slow table where they fit (the lanes of a
+  // quarter warp then read from different bank groups whatever rows they want),
+  // the table in global memory where not even one does
   const size_t one = sizeof(float) * kAdjRow * (size_t)a.slowRows;
-  a.tabCopies = 4;
+  a.tabCopies = 8;
   while (a.tabCopies > 1 && one * a.tabCopies > kAdjTableBytes) a.tabCopies /= 2;
   cudaError_t e;
   if (!doSlow) {
