@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(kSortMaxThreads)
   __shared__ int s_child[kMaxRanges];  // index of a split part among the split ones
   __shared__ int s_numNext, s_tie;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  admitSuccessor();
   for (int p = blockIdx.x; p < numPatches; p += gridDim.x) {
     const int n = rec[p].numAtoms, off = rec[p].bufferOffset;
     if (n <= 0) continue;  // block-uniform
@@ -107,24 +108,39 @@ __global__ void __launch_bounds__(kSortMaxThreads)
       for (int r = wib; r < nr; r += warps) {
         const int b = rb[r], e = re[r];
         const int sp = splitPoint(b, e);
-        double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+        // lows and negated highs: six minima over the warp. Lanes halve the
+        // values they hold step by step (3, 2 of 4, 1), so that 8 instead of 30
+        // values cross lanes; quantity 3 b16 + 2 b8 + b4 ends in the lanes of
+        // those bits
+        double v[6] = {1e300, 1e300, 1e300, 1e300, 1e300, 1e300};
         if (sp >= 0) {
           for (int k = b + lane; k < e; k += 32) {
             const int a = s_ord[k];
-            lo[0] = fmin(lo[0], s_x[a]);
-            hi[0] = fmax(hi[0], s_x[a]);
-            lo[1] = fmin(lo[1], s_y[a]);
-            hi[1] = fmax(hi[1], s_y[a]);
-            lo[2] = fmin(lo[2], s_z[a]);
-            hi[2] = fmax(hi[2], s_z[a]);
+            v[0] = fmin(v[0], s_x[a]);
+            v[1] = fmin(v[1], s_y[a]);
+            v[2] = fmin(v[2], s_z[a]);
+            v[3] = fmin(v[3], -s_x[a]);
+            v[4] = fmin(v[4], -s_y[a]);
+            v[5] = fmin(v[5], -s_z[a]);
           }
+        }
+        const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4;
+        double u[3];
 #pragma unroll
-          for (int o = 16; o >= 1; o >>= 1)
+        for (int q = 0; q < 3; ++q)
+          u[q] = fmin(b16 ? v[q + 3] : v[q], __shfl_xor_sync(0xffffffffu, b16 ? v[q] : v[q + 3], 16));
+        double w0 = fmin(b8 ? u[2] : u[0], __shfl_xor_sync(0xffffffffu, b8 ? u[0] : u[2], 8));
+        const double w1o = __shfl_xor_sync(0xffffffffu, u[1], 8);
+        const double w1 = b8 ? w0 : fmin(u[1], w1o);
+        double m = fmin(b4 ? w1 : w0, __shfl_xor_sync(0xffffffffu, b4 ? w0 : w1, 4));
+        m = fmin(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        m = fmin(m, __shfl_xor_sync(0xffffffffu, m, 1));
+        double lo[3], hi[3];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-              hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-            }
+        for (int d = 0; d < 3; ++d) {
+          const int src = 8 * (d >> 1) + 4 * (d & 1);
+          lo[d] = __shfl_sync(0xffffffffu, m, src);
+          hi[d] = -__shfl_sync(0xffffffffu, m, 16 + src);
         }
         if (lane == 0) {
           int axis = 0;
@@ -228,6 +244,7 @@ __global__ void computePositionsKernel(int numPatches, const nbk_local_record* _
                                        const double* __restrict__ px, const double* __restrict__ py,
                                        const double* __restrict__ pz,
                                        const float* __restrict__ charge, float4* __restrict__ xyzq) {
+  waitForPredecessor();
   for (int p = blockIdx.x; p < numPatches; p += gridDim.x) {
     const int n = rec[p].numAtoms, off = rec[p].bufferOffset, offNB = rec[p].bufferOffsetNBPad;
     const int npad = rec[p].numAtomsNBPad;
@@ -256,6 +273,8 @@ __global__ void updateVdwTypesExclDeviceKernel(int numPatches, const nbk_local_r
                                                int ljDim, int storage, int* __restrict__ vdwTypes,
                                                int* __restrict__ atomIndex, int2* __restrict__ excl,
                                                int* __restrict__ status) {
+  waitForPredecessor();
+  admitSuccessor();
   for (int p = blockIdx.x; p < numPatches; p += gridDim.x) {
     const int n = rec[p].numAtoms, off = rec[p].bufferOffset, offNB = rec[p].bufferOffsetNBPad;
     const int npad = rec[p].numAtomsNBPad;
@@ -286,6 +305,7 @@ __global__ void updateVdwTypesExclDeviceKernel(int numPatches, const nbk_local_r
 }
 
 __global__ void accumulateForcesKernel(const __grid_constant__ AccumulateArgs a) {
+  waitForPredecessor();
   for (int p = blockIdx.x; p < a.numPatches; p += gridDim.x) {
     const int n = a.rec[p].numAtoms, off = a.rec[p].bufferOffset, offNB = a.rec[p].bufferOffsetNBPad;
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
@@ -322,8 +342,7 @@ __global__ void accumulateForcesKernel(const __grid_constant__ AccumulateArgs a)
 
 cudaError_t launchAccumulateForces(const AccumulateArgs& a, cudaStream_t st) {
   if (a.numPatches <= 0) return cudaSuccess;
-  accumulateForcesKernel<<<min(a.numPatches, 65535), 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return launchOverlapped(accumulateForcesKernel, min(a.numPatches, 65535), 256, 0, st, a);
 }
 
 cudaError_t launchUpdateVdwTypesExclDevice(int numPatches, const nbk_local_record* rec,
@@ -332,10 +351,9 @@ cudaError_t launchUpdateVdwTypesExclDevice(int numPatches, const nbk_local_recor
                                            int storage, int* vdwTypes, int* atomIndex, int2* excl,
                                            int* status, cudaStream_t st) {
   if (numPatches <= 0) return cudaSuccess;
-  updateVdwTypesExclDeviceKernel<<<min(numPatches, 65535), 256, 0, st>>>(
-      numPatches, rec, vdw, gid, sortOrder, exclByAtom, numExclAtoms, ljDim, storage, vdwTypes,
-      atomIndex, excl, status);
-  return cudaGetLastError();
+  return launchOverlapped(updateVdwTypesExclDeviceKernel, min(numPatches, 65535), 256, 0, st, numPatches,
+                          rec, vdw, gid, sortOrder, exclByAtom, numExclAtoms, ljDim, storage, vdwTypes,
+                          atomIndex, excl, status);
 }
 
 }  // namespace nbk
@@ -381,10 +399,10 @@ extern "C" NBK_API int nbk_set_compute_positions(int numPatches, const nbk_local
   Lattice12 L;
   double* l = &L.ax;
   for (int k = 0; k < 12; ++k) l[k] = lattice[k];
-  computePositionsKernel<<<min(numPatches, 65535), 128, 0, (cudaStream_t)stream>>>(
-      numPatches, d_rec, reinterpret_cast<const double3*>(d_centre), L, d_sortOrder, chargeScaling,
-      d_x, d_y, d_z, d_charge, reinterpret_cast<float4*>(d_xyzq));
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launchOverlapped(
+      computePositionsKernel, min(numPatches, 65535), 128, 0, (cudaStream_t)stream, numPatches, d_rec,
+      reinterpret_cast<const double3*>(d_centre), L, d_sortOrder, chargeScaling, d_x, d_y, d_z,
+      d_charge, reinterpret_cast<float4*>(d_xyzq));
   if (e != cudaSuccess)
     return setLastError(NBK_ERR_CUDA,
                         std::string("nbk_set_compute_positions: ") + cudaGetErrorString(e));
