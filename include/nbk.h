@@ -217,8 +217,8 @@ NBK_API int nbk_build_tile_lists(nbk_handle h, int numPatches, int atomStorageSi
  * cancel to 1e-4 of the sum of |pair energies| only to ~1e-5. The LJ energy
  * (FP32 per pair) and the fast virial (from the fixed-point forces) hold
  * ~3e-7. Cost, measured on a B200 at 92,224 atoms (34 M pairs): the FP64
- * energy kernel runs 0.195 ms after the 0.403 ms force kernel, so an
- * evaluation with NBK_ENERGY costs about 1.5x a forces-only one. */
+ * energy kernel runs 0.207 ms after the 0.293 ms force kernel, so an
+ * evaluation with NBK_ENERGY costs about 1.8x one of forces only. */
 NBK_API int nbk_nonbonded_force(nbk_handle h, int atomStorageSize, unsigned flags,
                                 nbk_float3 lata, nbk_float3 latb, nbk_float3 latc,
                                 const nbk_float4* xyzq, int xyzqOnDevice, float cutoff2,
@@ -392,8 +392,10 @@ NBK_API int nbk_measure_fp64_peak(int deviceID, double* tflops);
  * Synchronises the stream; overwrites the handle's force and energy
  * accumulators, so call it before an evaluation, not between an evaluation
  * and its nbk_reduce_virial_energy. Untuned handles use 4 CTAs per SM and one
- * warp per list; the tuner keeps that default unless another shape is at
- * least 3% faster, since shapes are timed back to back on a warm L2. */
+ * warp per list, two or four where there are few lists; the tuner keeps that
+ * default unless another shape is at least 3% faster, since shapes are timed
+ * back to back on a warm L2. The warps per list also hold for the precise
+ * kernel. */
 NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* stream);
 
 /* The launch shape in use for a flag combination and the time per force

@@ -79,7 +79,7 @@ double erfOverR(double beta, double s) {
   if (s < 0.0 || beta * beta * s < 0.5) {
     const double x = -beta * beta * s;
     double term = 1.0, sum = 0.0;
-    for (int n = 0; n < 80; ++n) {
+    for (int n = 0; n < 80 && std::fabs(term) > 1e-20; ++n) {  // sum >= 0.8: the rest is lost in it
       sum += term / (2 * n + 1);
       term *= x / (n + 1);
     }
@@ -166,7 +166,7 @@ static double slowForceFactor(double beta, double rc, double s) {
   if (y < 0.5) {
     // -2 d/ds of erfOverR's series
     double term = 1.0, sum = 0.0;  // term: (-y)^(n-1)/(n-1)!
-    for (int n = 1; n < 80; ++n) {
+    for (int n = 1; n < 80 && std::fabs(term) > 1e-20; ++n) {
       sum += term / (2 * n + 1);
       term *= -y / n;
     }

@@ -357,6 +357,75 @@ __global__ void gatherKernel(const __grid_constant__ GatherArgs a) {
   }
 }
 
+// The same with `order` lanes per atom (orders 4 and 8), each on one x of the
+// stencil: a row of it is then one or two 32-byte sectors of one load, where a
+// thread per atom makes every load touch 32 sectors; those accesses bound the
+// kernel, not the weights that the lanes of an atom form together. Each lane
+// sums its column in a fixed order (along y, then z), and the lanes' sums are
+// added by a fixed butterfly.
+template <int order>
+__global__ void __launch_bounds__(128) gatherColumnsKernel(const __grid_constant__ GatherArgs a) {
+  constexpr int kAtoms = 32 / order;  // atoms per warp
+  const int lane = threadIdx.x & 31;
+  const int x0 = lane % order;
+  const int warpsTotal = (gridDim.x * blockDim.x) >> 5;
+  const int K12 = a.K1 * a.K2;  // grid indices below 2^31 (checked at creation)
+  for (int a0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kAtoms; a0 < a.n;
+       a0 += warpsTotal * kAtoms) {  // warp-uniform
+    const int i = a0 + lane / order;
+    const float4 at = a.atoms[min(i, a.n - 1)];
+    int ix, iy, iz;
+    float wx, wy, wz;
+    gridCell(at, a.K1, a.K2, a.K3, ix, iy, iz, wx, wy, wz);
+    float tx[order], ty[order], tz[order], dx[order], dy[order], dz[order];
+    bsplineThetaD<order>(wx, tx, dx);
+    bsplineThetaD<order>(wy, ty, dy);
+    bsplineThetaD<order>(wz, tz, dz);
+    float txl = 0.f, dxl = 0.f;
+#pragma unroll
+    for (int k = 0; k < order; ++k) {
+      txl = k == x0 ? tx[k] : txl;
+      dxl = k == x0 ? dx[k] : dxl;
+    }
+    const float* column = a.grid + (ix + x0 >= a.K1 ? ix + x0 - a.K1 : ix + x0);
+    int rows[order];
+#pragma unroll
+    for (int y0 = 0; y0 < order; ++y0)
+      rows[y0] = a.K1 * (iy + y0 >= a.K2 ? iy + y0 - a.K2 : iy + y0);
+    float f1 = 0.f, f2 = 0.f, f3 = 0.f;
+#pragma unroll
+    for (int z0 = 0; z0 < order; ++z0) {
+      const float* plane = column + K12 * (iz + z0 >= a.K3 ? iz + z0 - a.K3 : iz + z0);
+      float s = 0.f, sd = 0.f;  // the column's sums of theta_y g and dtheta_y g
+#pragma unroll
+      for (int y0 = 0; y0 < order; ++y0) {
+        const float g = __ldg(plane + rows[y0]);
+        s = fmaf(ty[y0], g, s);
+        sd = fmaf(dy[y0], g, sd);
+      }
+      f1 = fmaf(s, tz[z0], f1);
+      f2 = fmaf(sd, tz[z0], f2);
+      f3 = fmaf(s, dz[z0], f3);
+    }
+    f1 *= dxl;
+    f2 *= txl;
+    f3 *= txl;
+#pragma unroll
+    for (int o = 1; o < order; o <<= 1) {
+      f1 += __shfl_xor_sync(0xffffffffu, f1, o);
+      f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+      f3 += __shfl_xor_sync(0xffffffffu, f3, o);
+    }
+    if (i < a.n && x0 == 0) {
+      const double q = -(double)at.w;
+      const double g1 = q * f1 * a.K1, g2 = q * f2 * a.K2, g3 = q * f3 * a.K3;
+      a.force[i] = make_float3((float)(g1 * a.r[0] + g2 * a.r[3] + g3 * a.r[6]),
+                               (float)(g1 * a.r[1] + g2 * a.r[4] + g3 * a.r[7]),
+                               (float)(g1 * a.r[2] + g2 * a.r[5] + g3 * a.r[8]));
+    }
+  }
+}
+
 __global__ void atomsFromPositionsKernel(int n, const double* __restrict__ x,
                                          const double* __restrict__ y, const double* __restrict__ z,
                                          const float* __restrict__ charge, double qscale, Recip R,
@@ -632,11 +701,13 @@ extern "C" NBK_API int nbk_pme_gather_force(nbk_pme p, int n, const nbk_float4* 
   a.grid = p->gridReal;
   a.force = reinterpret_cast<float3*>(force);
   const int blocks = std::min((n + 127) / 128, p->numSM * 16);
+  // four warps of 32 / order atoms each
+  const int perBlock = 128 / p->order, columns = std::min((n + perBlock - 1) / perBlock, p->numSM * 32);
   cudaStream_t st = (cudaStream_t)stream;
   switch (p->order) {
-    case 4: gatherKernel<4><<<blocks, 128, 0, st>>>(a); break;
+    case 4: gatherColumnsKernel<4><<<columns, 128, 0, st>>>(a); break;
     case 6: gatherKernel<6><<<blocks, 128, 0, st>>>(a); break;
-    default: gatherKernel<8><<<blocks, 128, 0, st>>>(a); break;
+    default: gatherColumnsKernel<8><<<columns, 128, 0, st>>>(a); break;
   }
   PME_CUDA(cudaGetLastError(), "nbk_pme_gather_force");
   return NBK_OK;
