@@ -307,7 +307,7 @@ struct GatherArgs {
   float3* force;
 };
 
-// One thread per atom: the gradient of the interpolated potential, summed
+// One thread per atom (order 6): the gradient of the interpolated potential, summed
 // over the order^3 points in a fixed order (along x first, then row by row),
 // then -q times the Cartesian gradient.
 template <int order>
@@ -362,7 +362,11 @@ __global__ void gatherKernel(const __grid_constant__ GatherArgs a) {
 // thread per atom makes every load touch 32 sectors; those accesses bound the
 // kernel, not the weights that the lanes of an atom form together. Each lane
 // sums its column in a fixed order (along y, then z), and the lanes' sums are
-// added by a fixed butterfly.
+// added by a fixed butterfly: the rounding errors are no larger than along x
+// first (order 4 the same within 20%, order 8 15-45% smaller, on smooth fields
+// against 64 bits). Order 4, against the thread per atom: 92k atoms on 108 x 108
+// x 80 points 10.9 -> 9.2 us, 1.07M on 225^3 83.7 -> 65.7 us. Order 6 does not
+// divide the warp and keeps the thread per atom.
 template <int order>
 __global__ void __launch_bounds__(128) gatherColumnsKernel(const __grid_constant__ GatherArgs a) {
   constexpr int kAtoms = 32 / order;  // atoms per warp
