@@ -923,7 +923,10 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
     cudaError_t e = dTo.ensure(cnt[0]);
     if (e == cudaSuccess) e = dJatom.ensure(std::max(next, 1));
     if (e == cudaSuccess) e = dExcl.ensure(std::max(next, 1));
-    if (e == cudaSuccess) e = cudaMemcpy(dTo.p, to.data(), sizeof(int) * cnt[0], cudaMemcpyHostToDevice);
+    // on the kernel's stream: a copy from pageable memory may return before it
+    // has landed, and a non-blocking stream does not wait for the default one
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(dTo.p, to.data(), sizeof(int) * cnt[0], cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
       e = launchExportTiles(cnt[0], h->refinedLists(), dTo.p, h->jatom2.p, h->excl2.p, dJatom.p,
                             dExcl.p, st);
