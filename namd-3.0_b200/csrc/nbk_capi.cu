@@ -386,14 +386,14 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   };
   fin(h->ljTable.ensure(dim * dim), "nbk_create: alloc");
   fin(h->ljExclTable.ensure(dim * dim), "nbk_create: alloc");
-  if (rc == NBK_OK) fin(cudaMemcpy(h->ljTable.p, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
-  if (rc == NBK_OK) fin(cudaMemcpy(h->ljExclTable.p, te.data(), sizeof(float2) * te.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+  if (rc == NBK_OK) fin(uploadNow(h->ljTable.p, t.data(), sizeof(float2) * t.size()), "nbk_create: copy");
+  if (rc == NBK_OK) fin(uploadNow(h->ljExclTable.p, te.data(), sizeof(float2) * te.size()), "nbk_create: copy");
   // FP64 slow-term table over s in [0, pairlistdist^2 + 2]: the runtime cutoff
   // can be anything up to the pairlist cutoff
   std::vector<double> slow;
   h->slowTableRows = buildSlowTable(p->ewaldcof, p->cutoff, p->pairlistdist, slow, &h->slowStep);
   fin(h->slowTable.ensure(slow.size() / 2), "nbk_create: alloc");
-  if (rc == NBK_OK) fin(cudaMemcpy(h->slowTable.p, slow.data(), sizeof(double) * slow.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+  if (rc == NBK_OK) fin(uploadNow(h->slowTable.p, slow.data(), sizeof(double) * slow.size()), "nbk_create: copy");
   std::vector<float4> at(2 * (size_t)h->slowTableRows);
   for (int k = 0; k < h->slowTableRows; ++k) {
     const double* r = &slow[(size_t)k * kSlowTableRow];
@@ -401,7 +401,7 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
     at[2 * k + 1] = make_float4((float)r[4], (float)r[5], 0.f, 0.f);
   }
   fin(h->adjTable.ensure(at.size()), "nbk_create: alloc");
-  if (rc == NBK_OK) fin(cudaMemcpy(h->adjTable.p, at.data(), sizeof(float4) * at.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+  if (rc == NBK_OK) fin(uploadNow(h->adjTable.p, at.data(), sizeof(float4) * at.size()), "nbk_create: copy");
   std::vector<float4> ft;
   double ftStep = 1.0;
   h->pk.tabRows = buildForceTable(p->ewaldcof, p->cutoff, p->pairlistdist, ft, &ftStep);
@@ -409,7 +409,7 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   h->pk.tabInvStep = (float)(1.0 / ftStep);
   if (h->pk.tabRows > 0) {
     fin(h->forceTable.ensure(ft.size()), "nbk_create: alloc");
-    if (rc == NBK_OK) fin(cudaMemcpy(h->forceTable.p, ft.data(), sizeof(float4) * ft.size(), cudaMemcpyHostToDevice), "nbk_create: copy");
+    if (rc == NBK_OK) fin(uploadNow(h->forceTable.p, ft.data(), sizeof(float4) * ft.size()), "nbk_create: copy");
     h->pk.tab = h->forceTable.p;
   }
   fin(h->acc.ensure(kAccCount), "nbk_create: alloc");
@@ -417,6 +417,7 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   fin(h->ve.ensure(1), "nbk_create: alloc");
   if (rc == NBK_OK) fin(cudaMemset(h->acc.p, 0, sizeof(long long) * kAccCount), "nbk_create: memset");
   if (rc == NBK_OK) fin(cudaMemset(h->counters.p, 0, sizeof(int) * 8), "nbk_create: memset");
+  if (rc == NBK_OK) fin(cudaStreamSynchronize(cudaStreamLegacy), "nbk_create: memset");
   if (rc != NBK_OK) {
     nbk_destroy(h);
     return rc;
@@ -504,7 +505,7 @@ NBK_API int nbk_bind_exclusions(nbk_handle h, int numExclusions, const unsigned 
     return setErr(NBK_ERR_ARG, "nbk_bind_exclusions: bad argument");
   NBK_CUDA(h->exclBits.ensure(std::max(numExclusions, 1)), "nbk_bind_exclusions");
   if (numExclusions)
-    NBK_CUDA(cudaMemcpy(h->exclBits.p, bits, sizeof(unsigned) * numExclusions, cudaMemcpyHostToDevice),
+    NBK_CUDA(uploadNow(h->exclBits.p, bits, sizeof(unsigned) * numExclusions),
              "nbk_bind_exclusions");
   h->numExclWords = numExclusions;
   return NBK_OK;
@@ -1056,13 +1057,13 @@ NBK_API int nbk_set_replicas(nbk_handle h, int numReplicas, const int* repOfComp
   NBK_CUDA(h->repLJExcl.ensure(te.size()), "nbk_set_replicas");
   NBK_CUDA(h->acc.ensure((size_t)kAccCount * numReplicas), "nbk_set_replicas");
   NBK_CUDA(h->ve.ensure(numReplicas), "nbk_set_replicas");
-  NBK_CUDA(cudaMemcpy(h->compRep.p, repOfCompute, sizeof(int) * h->numComputes, cudaMemcpyHostToDevice),
+  NBK_CUDA(uploadNow(h->compRep.p, repOfCompute, sizeof(int) * h->numComputes),
            "nbk_set_replicas");
-  if (n) NBK_CUDA(cudaMemcpy(h->slotRep.p, slotRep.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "nbk_set_replicas");
-  NBK_CUDA(cudaMemcpy(h->repLat.p, lattices, sizeof(float3) * 3 * (size_t)numReplicas, cudaMemcpyHostToDevice),
+  if (n) NBK_CUDA(uploadNow(h->slotRep.p, slotRep.data(), sizeof(int) * n), "nbk_set_replicas");
+  NBK_CUDA(uploadNow(h->repLat.p, lattices, sizeof(float3) * 3 * (size_t)numReplicas),
            "nbk_set_replicas");
-  NBK_CUDA(cudaMemcpy(h->repLJ.p, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice), "nbk_set_replicas");
-  NBK_CUDA(cudaMemcpy(h->repLJExcl.p, te.data(), sizeof(float2) * te.size(), cudaMemcpyHostToDevice),
+  NBK_CUDA(uploadNow(h->repLJ.p, t.data(), sizeof(float2) * t.size()), "nbk_set_replicas");
+  NBK_CUDA(uploadNow(h->repLJExcl.p, te.data(), sizeof(float2) * te.size()),
            "nbk_set_replicas");
   NBK_CUDA(cudaMemsetAsync(h->acc.p, 0, sizeof(long long) * kAccCount * (size_t)numReplicas, st),
            "nbk_set_replicas");
@@ -1379,7 +1380,7 @@ NBK_API int nbk_set_exclusions_by_atom(nbk_handle h, int numAtoms, const nbk_int
   if (rc) return rc;
   if (numAtoms <= 0 || !hx) return setErr(NBK_ERR_ARG, "nbk_set_exclusions_by_atom: bad argument");
   NBK_CUDA(h->exclByAtom.ensure(numAtoms), "nbk_set_exclusions_by_atom");
-  NBK_CUDA(cudaMemcpy(h->exclByAtom.p, hx, sizeof(int2) * numAtoms, cudaMemcpyHostToDevice),
+  NBK_CUDA(uploadNow(h->exclByAtom.p, hx, sizeof(int2) * numAtoms),
            "nbk_set_exclusions_by_atom");
   h->numExclByAtom = numAtoms;
   return NBK_OK;

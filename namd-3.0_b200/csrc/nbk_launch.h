@@ -29,6 +29,14 @@ cudaError_t launchOverlapped(void (*kernel)(P...), int blocks, int threads, size
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Copies host data up and returns once it has landed: a copy from pageable
+// memory may return before that, and the caller's next stream need not wait for
+// the default one.
+inline cudaError_t uploadNow(void* dst, const void* src, size_t bytes) {
+  const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // Zeroes the 64-bit words a[0, na), b[0, nb) and the 32-bit words c[0, nc),
 // d[0, nd) in one launch (memsets cost a gap each).
 cudaError_t launchClear(long long* a, size_t na, long long* b, size_t nb, int* c, int nc, int* d,

@@ -698,11 +698,11 @@ extern "C" NBK_API int nbk_pme_create(int deviceID, const nbk_pme_grid* g, doubl
     bModuli(p->K1, p->order, b1);
     bModuli(p->K2, p->order, b2);
     bModuli(p->K3, p->order, b3);
-    e = cudaMemcpy(p->bm, b1.data(), sizeof(float) * p->K1, cudaMemcpyHostToDevice);
+    e = uploadNow(p->bm, b1.data(), sizeof(float) * p->K1);
     if (e == cudaSuccess)
-      e = cudaMemcpy(p->bm + p->K1, b2.data(), sizeof(float) * p->K2, cudaMemcpyHostToDevice);
+      e = uploadNow(p->bm + p->K1, b2.data(), sizeof(float) * p->K2);
     if (e == cudaSuccess)
-      e = cudaMemcpy(p->bm + p->K1 + p->K2, b3.data(), sizeof(float) * p->K3, cudaMemcpyHostToDevice);
+      e = uploadNow(p->bm + p->K1 + p->K2, b3.data(), sizeof(float) * p->K3);
   }
   if (e != cudaSuccess) {
     nbk_pme_destroy(p);
