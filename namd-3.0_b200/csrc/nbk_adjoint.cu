@@ -313,13 +313,12 @@ __global__ void adjointOutKernel(int n, const long long* __restrict__ g, int str
 
 template <bool S, bool SH>
 static cudaError_t launchAdj(const AdjArgs& a, size_t shmem, int numSM, cudaStream_t st) {
+  static KernelLimits limits;
   auto k = adjointKernel<S, SH>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
+  int blocks = 0;
+  const cudaError_t e = limits.blocksPerSM(k, kAdjThreads, shmem, &blocks);
   if (e != cudaSuccess) return e;
-  int nb = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kAdjThreads, shmem);
-  if (e != cudaSuccess) return e;
-  k<<<numSM * (nb > 0 ? nb : 1), kAdjThreads, shmem, st>>>(a);
+  k<<<numSM * blocks, kAdjThreads, shmem, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -26,8 +26,6 @@
 #include "nbk_internal.cuh"
 #include "nbk_launch.h"
 
-#include <mutex>
-
 namespace nbk {
 
 constexpr int kForceWarps = 4;
@@ -829,41 +827,12 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
   flushPrecise<doEnergy>(a.acc + (size_t)curRep * kAccCount, lane, accQ, npair);
 }
 
-// Blocks per SM of one kernel instance on one device for one dynamic
-// shared-memory size, with the opt-in set on that device; looked up once per
-// (device, size) and kept per instance, under a lock, so handles on different
-// devices or threads neither share a stale entry nor race.
-constexpr int kMaxDevicesCached = 64;
-struct OccCache {
-  std::mutex mu;
-  size_t shmem[kMaxDevicesCached];
-  int blocks[kMaxDevicesCached];
-  OccCache() {
-    for (int d = 0; d < kMaxDevicesCached; ++d) shmem[d] = (size_t)-1, blocks[d] = 0;
-  }
-};
-
 template <typename K>
-static cudaError_t launchPersistent(K kernel, OccCache& cache, int threads, size_t shmem,
+static cudaError_t launchPersistent(K kernel, KernelLimits& limits, int threads, size_t shmem,
                                     int numSM, cudaStream_t st, const ForceArgs& a) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= kMaxDevicesCached) return cudaErrorInvalidDevice;
   int blocks = 0;
-  {
-    std::lock_guard<std::mutex> lock(cache.mu);
-    if (cache.shmem[dev] != shmem) {
-      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
-      if (e != cudaSuccess) return e;
-      int nb = 0;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, shmem);
-      if (e != cudaSuccess) return e;
-      cache.blocks[dev] = nb > 0 ? nb : 1;
-      cache.shmem[dev] = shmem;
-    }
-    blocks = cache.blocks[dev];
-  }
+  const cudaError_t e = limits.blocksPerSM(kernel, threads, shmem, &blocks);
+  if (e != cudaSuccess) return e;
   return launchOverlapped(kernel, numSM * blocks, threads, shmem, st, a);
 }
 
@@ -874,17 +843,17 @@ static cudaError_t launchT(const ForceArgs& a, int numSM, cudaStream_t st) {
     if (a.pk.tabRows > 0) {
       // as many copies of the table as fit in kForceTableBytes, up to the 8 that
       // keep quarter warps free of bank conflicts
-      static OccCache cache;
+      static KernelLimits limits;
       ForceArgs t = a;
       const size_t one = sizeof(float4) * (size_t)a.pk.tabRows;
       t.tabCopies = 8;
       while (t.tabCopies > 1 && one * t.tabCopies > kForceTableBytes) t.tabCopies /= 2;
-      return launchPersistent(forceKernel<E, V, S, true, B, MINB>, cache, kForceThreads,
+      return launchPersistent(forceKernel<E, V, S, true, B, MINB>, limits, kForceThreads,
                               one * t.tabCopies + lj, numSM, st, t);
     }
   }
-  static OccCache cache;
-  return launchPersistent(forceKernel<E, V, S, false, B, MINB>, cache, kForceThreads, lj, numSM,
+  static KernelLimits limits;
+  return launchPersistent(forceKernel<E, V, S, false, B, MINB>, limits, kForceThreads, lj, numSM,
                           st, a);
 }
 
@@ -934,10 +903,10 @@ bool needsPrecise(unsigned flags) {
 
 template <bool E, bool V, bool S, bool B, int C>
 static cudaError_t launchPC(const ForceArgs& a, int numSM, cudaStream_t st) {
-  static OccCache cache;
+  static KernelLimits limits;
   const size_t shmem = (S && C > 0) ? sizeof(double) * kSlowTableDeg1 * (size_t)a.slowTableRows * C
                                     : 0;
-  return launchPersistent(preciseKernel<E, V, S, B, C>, cache, kPreciseThreads, shmem, numSM, st,
+  return launchPersistent(preciseKernel<E, V, S, B, C>, limits, kPreciseThreads, shmem, numSM, st,
                           a);
 }
 

@@ -3,12 +3,74 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "nbk_internal.cuh"
 
 namespace nbk {
+
+// Dynamic shared memory and occupancy of one kernel instance, per device. Handles
+// on several host threads launch one instance with different sizes at once, so
+// the limit is only ever raised: a launch that follows outside the lock finds at
+// least what it asked for. Occupancy is looked up once for each of the sizes
+// last in use.
+class KernelLimits {
+ public:
+  template <typename K>
+  cudaError_t allow(K kernel, size_t shmem) {
+    int dev = 0;
+    const cudaError_t e = device(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    return raise(kernel, dev, shmem);
+  }
+  template <typename K>
+  cudaError_t blocksPerSM(K kernel, int threads, size_t shmem, int* blocks) {
+    int dev = 0;
+    cudaError_t e = device(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    PerDevice& d = devices[dev];
+    for (int k = 0; k < kSizes; ++k)
+      if (d.blocks[k] > 0 && d.shmem[k] == shmem) {
+        *blocks = d.blocks[k];
+        return cudaSuccess;
+      }
+    e = raise(kernel, dev, shmem);
+    int nb = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, shmem);
+    if (e != cudaSuccess) return e;
+    d.shmem[d.next] = shmem;
+    *blocks = d.blocks[d.next] = nb > 0 ? nb : 1;
+    d.next = (d.next + 1) % kSizes;
+    return cudaSuccess;
+  }
+
+ private:
+  static constexpr int kDevices = 64, kSizes = 8;
+  struct PerDevice {
+    size_t allowed = 0;
+    size_t shmem[kSizes] = {};
+    int blocks[kSizes] = {};  // 0: free
+    int next = 0;
+  };
+  static cudaError_t device(int* dev) {
+    const cudaError_t e = cudaGetDevice(dev);
+    return e != cudaSuccess ? e : (*dev < 0 || *dev >= kDevices) ? cudaErrorInvalidDevice : cudaSuccess;
+  }
+  template <typename K>
+  cudaError_t raise(K kernel, int dev, size_t shmem) {
+    if (shmem <= devices[dev].allowed) return cudaSuccess;
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
+    if (e == cudaSuccess) devices[dev].allowed = shmem;
+    return e;
+  }
+  std::mutex mu;
+  PerDevice devices[kDevices];
+};
 
 // Launches a kernel that may be scheduled while the kernel before it in the
 // stream still runs; it calls waitForPredecessor before it uses anything that

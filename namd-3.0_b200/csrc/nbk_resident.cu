@@ -371,8 +371,8 @@ extern "C" NBK_API int nbk_sort_patch_atoms(int numPatches, const nbk_local_reco
                                          std::to_string(NBK_MAX_PATCH_ATOMS));
   if (numPatches == 0) return NBK_OK;
   const size_t smem = (size_t)maxPatchAtoms * (4 * sizeof(double) + 5 * sizeof(int));
-  cudaError_t e = cudaFuncSetAttribute(sortPatchAtomsKernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static KernelLimits limits;
+  cudaError_t e = limits.allow(sortPatchAtomsKernel, smem);
   if (e == cudaSuccess) {
     // a thread per atom of the largest patch where a block can have as many
     const int threads = std::min(kSortMaxThreads, std::max(64, (maxPatchAtoms + 31) / 32 * 32));

@@ -21,6 +21,18 @@ def mixed_box(seed=2, natoms=20000, frac=0.3, box=None):
     return nbk.System(nbk.NBK_SYS_MIXED, seed, natoms, frac, box=box)
 
 
+def wider_lj(lj, types):
+    """An LJ table (dim, A, B, A14, B14) within one of more types, none of which
+    an atom has."""
+    dim = lj[0]
+    out = [types]
+    for t in lj[1:]:
+        w = np.zeros((types, types))
+        w[:dim, :dim] = np.asarray(t).reshape(dim, dim)
+        out.append(w.reshape(-1))
+    return tuple(out)
+
+
 def rms_rel(a, b):
     num = np.sqrt(((a - b) ** 2).sum())
     den = np.sqrt((b ** 2).sum())
