@@ -195,7 +195,9 @@ NBK_API int nbk_build_tile_lists(nbk_handle h, int numPatches, int atomStorageSi
 
 /* CudaComputeNonbondedKernel::nonbondedForce, src/CudaComputeNonbondedKernel.cu:2076-3590.
  * flags = NBK_ENERGY|NBK_VIRIAL|NBK_SLOW|NBK_PAIRLIST|NBK_CORRECTIONS.
- * xyzq as for nbk_build_tile_lists (NULL = reuse the build's positions).
+ * xyzq as for nbk_build_tile_lists (NULL = reuse the build's positions). cutoff2
+ * may be anything up to the build's plcutoff2, also beyond params.pairlistdist:
+ * the slow terms then come from their formulas instead of their tables.
  * Forces are accumulated deterministically as 64-bit fixed point (2^32 per
  * kcal/mol/A) and then written as float4 to any non-NULL output:
  *   d_forces / d_forcesSlow : device float4[atomStorageSize] (w = 0)
@@ -259,7 +261,8 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
  * for the last refined tile lists and the bound positions (call after an
  * nbk_nonbonded_force of the same positions): with respect to the positions
  * (a Hessian-vector product), the scaled charges xyzq.w, and the scaled LJ
- * table entries. Pair terms are recomputed from the tile lists; nothing of
+ * table entries. Takes the pairs within params.cutoff, whatever cutoff2 the
+ * evaluation was given. Pair terms are recomputed from the tile lists; nothing of
  * the forward pass is stored. wS and cS are used with NBK_SLOW in flags.
  *   d_wF, d_wS   : device float4[atomStorageSize] cotangents (w ignored)
  *   h_typeMask   : host int[vdwTableDim]; LJ gradients are accumulated for
@@ -335,7 +338,8 @@ NBK_API const char* nbk_noalloc_last_error(void);
  * s = r^2, on s in [k D - D/2, k D + D/2], as coefficients c0..c5 of powers of
  * (s - k D).
  * The slow pair energy is qq phi_s(s), the slow force factor
- * (dE/dr)/r = 2 qq phi_s'(s). Rows cover s up to pairlistdist^2 + 2.
+ * (dE/dr)/r = 2 qq phi_s'(s). Rows cover s up to pairlistdist^2 + 2; beyond, the
+ * kernel evaluates the formula.
  * Host-only (no GPU needed): returns the number of rows and, when out is not
  * NULL, writes them (maxRows must be at least that number); step may be NULL;
  * NBK_ERR_ARG for bad parameters. */

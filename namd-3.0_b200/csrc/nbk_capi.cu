@@ -248,6 +248,12 @@ int splitOf(const nbk_context* h, int key) {
   return h->numLists >= 7 * warps ? 0 : h->numLists >= 3 * warps ? 1 : 2;
 }
 
+// The slow-term tables reach pairlistdist^2 + 2, but a caller may build its lists
+// for a larger distance and evaluate up to there.
+bool beyondTables(const nbk_context* h, float cutoff2) {
+  return (double)cutoff2 > h->prm.pairlistdist * h->prm.pairlistdist + 2.0;
+}
+
 // Force-kernel arguments for the handle's compacted lists, positions, lattice,
 // constants and replicas.
 ForceArgs refinedForceArgs(nbk_context* h, float cutoff2) {
@@ -273,6 +279,7 @@ ForceArgs refinedForceArgs(nbk_context* h, float cutoff2) {
   a.slowTableRows = h->slowTableRows;
   a.slowStep = h->slowStep;
   a.slowInvStep = 1.0 / h->slowStep;
+  a.beyondTables = beyondTables(h, cutoff2);
   if (h->nrep > 0) {
     a.compRep = h->compRep.p;
     a.repLat = h->repLat.p;

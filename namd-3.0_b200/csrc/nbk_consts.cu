@@ -177,7 +177,7 @@ static double slowForceFactor(double beta, double rc, double s) {
 }
 
 // The force kernel's FP32 table of the slow force factor over s in [0,
-// pairlistdist^2 + 2] (the runtime cutoff is at most the pairlist cutoff): the
+// pairlistdist^2 + 2] (evaluations with a larger cutoff take the erfc form): the
 // step starts at 32 A^2 and is halved until the fit is within kForceTableTol of
 // the factor's largest value or the table would pass kForceTableMaxRows. Returns the
 // number of rows, 0 when the tolerance asks for more than that.

@@ -123,19 +123,31 @@ struct LaneSums {
 // copy c at s_slowTab[(k * P + n) * kCopies + c] with P = kSlowTableDeg1 / 2;
 // lane l reads copy l % kCopies, so with 8 copies the 8 lanes of a quarter
 // warp (one 16-byte bank group each) never conflict, whatever rows they read.
-// kCopies == 0: the global copy (kSlowTableRow doubles per row).
+// kCopies == 0: the global copy (kSlowTableRow doubles per row); kBeyond: the
+// same, with pairs beyond the table from the formula.
+constexpr int kBeyond = -1;
 extern __shared__ __align__(16) double2 s_slowTab[];
 
 struct SlowTable {
   const double2* gl;
   unsigned last;
   double step, invStep;
+  double sMax;  // centre of the last row
 };
+
+// phi_s and phi_s' from the formula, for pairs beyond the table: with E = erf(beta
+// r)/r and G = 2 beta/sqrt(pi) e^{-beta^2 s}, E' = (G - E)/(2 s). Out of line: few
+// evaluations reach there.
+__device__ __noinline__ double2 slowTermsDirect(const NbkConst& c, const double s) {
+  const double r = sqrt(s), E = erf(c.betad * r) / r;
+  const double G = c.betad * 1.1283791670955126 * exp(-c.betad * c.betad * s);  // 2/sqrt(pi)
+  return make_double2(fma(c.hBd, s, c.hAd) - E, c.hBd - (G - E) / (2.0 * s));
+}
 
 template <int kCopies>
 __device__ __forceinline__ double2 slowPair(const SlowTable& T, const unsigned k, const int n,
                                             const int lane) {
-  if (kCopies > 0) {
+  if constexpr (kCopies > 0) {
     return s_slowTab[(k * (kSlowTableDeg1 / 2) + n) * kCopies + (lane & (kCopies - 1))];
   } else {
     return __ldg(T.gl + (size_t)k * (kSlowTableRow / 2) + n);
@@ -155,7 +167,11 @@ __device__ __forceinline__ void precisePair(const PairTerms& u, const SlowTable&
                                             const NbkConst& c, const int lane, LaneSums& L) {
   const double s = fma(u.dz, u.dz, fma(u.dy, u.dy, u.dx * u.dx));
   double p = 0.0, dp = 0.0;
-  if (doSlow) {
+  if (doSlow && kCopies == kBeyond && s > T.sMax) {
+    const double2 d = slowTermsDirect(c, s);
+    p = d.x;
+    dp = d.y;
+  } else if (doSlow) {
     // row k = nearest integer to s/D: adding 1.5 * 2^52 rounds s/D (exact, D
     // a power of two) into the low word; k is clamped to the last row (any
     // bit pattern stays in the table) and w = s - k D
@@ -750,6 +766,7 @@ __global__ void __launch_bounds__(kPreciseThreads, kPreciseMinBlocks)
   T.step = a.slowStep;
   T.invStep = a.slowInvStep;
   T.gl = a.slowTable;
+  T.sMax = a.slowStep * (double)(a.slowTableRows - 1);
   if (doSlow && kCopies > 0) {
     constexpr int P = kSlowTableDeg1 / 2;
     for (int k = threadIdx.x; k < P * a.slowTableRows * kCopies; k += blockDim.x) {
@@ -840,7 +857,7 @@ template <bool E, bool V, bool S, bool B, int MINB>
 static cudaError_t launchT(const ForceArgs& a, int numSM, cudaStream_t st) {
   const size_t lj = B ? 0 : sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
   if constexpr (S) {
-    if (a.pk.tabRows > 0) {
+    if (a.pk.tabRows > 0 && !a.beyondTables) {  // the erfc form has no end
       // as many copies of the table as fit in kForceTableBytes, up to the 8 that
       // keep quarter warps free of bank conflicts
       static KernelLimits limits;
@@ -911,9 +928,11 @@ static cudaError_t launchPC(const ForceArgs& a, int numSM, cudaStream_t st) {
 }
 
 // the table in shared memory with 8 interleaved copies when they fit in 40 KB
-// (106 rows), else read from global memory
+// (106 rows), else read from global memory; beyond its reach the instance that
+// can go on from there
 template <bool E, bool V, bool S, bool B>
 static cudaError_t launchP(const ForceArgs& a, int numSM, cudaStream_t st) {
+  if (S && a.beyondTables) return launchPC<E, V, S, B, S ? kBeyond : 0>(a, numSM, st);
   if (sizeof(double) * kSlowTableDeg1 * (size_t)a.slowTableRows * 8 <= 40 * 1024)
     return launchPC<E, V, S, B, 8>(a, numSM, st);
   return launchPC<E, V, S, B, 0>(a, numSM, st);

@@ -410,6 +410,7 @@ struct ForceArgs {
   const double2* slowTable;    // [slowTableRows * kSlowTableRow / 2] phi_s rows (FP64)
   int slowTableRows;
   double slowStep, slowInvStep;  // table step D (a power of two) and 1/D
+  bool beyondTables;           // the cutoff exceeds the distance the tables were built for
   unsigned* liveOut;           // [numJtiles][32] interacting-pair words (force kernel writes,
                                // precise kernel reads), block order
   // replicas (batched evaluation; all NULL for a single system)
