@@ -261,7 +261,9 @@ NBK_API int nbk_export_tile_lists(nbk_handle h, int* numTileLists, int* numJtile
  * for the last refined tile lists and the bound positions (call after an
  * nbk_nonbonded_force of the same positions): with respect to the positions
  * (a Hessian-vector product), the scaled charges xyzq.w, and the scaled LJ
- * table entries. Takes the pairs within params.cutoff, whatever cutoff2 the
+ * table entries. d_gradFixed and d_gradXQ are the same bits in every call on one
+ * layout (i sums are FP32 over a list or, where there are few, a part of one by a
+ * fixed rule), d_gradAB to the rounding of FP64 sums in any order. Takes the pairs within params.cutoff, whatever cutoff2 the
  * evaluation was given. Pair terms are recomputed from the tile lists; nothing of
  * the forward pass is stored. wS and cS are used with NBK_SLOW in flags.
  *   d_wF, d_wS   : device float4[atomStorageSize] cotangents (w ignored)

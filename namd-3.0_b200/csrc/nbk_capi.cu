@@ -237,15 +237,18 @@ int tuneKey(const nbk_context* h, unsigned flags) {
          ((flags & NBK_SLOW) ? 1 : 0);
 }
 
-// Work items per tile list (log2) unless the tuner or the caller chose. A list
-// is one warp's work, about 3 us per tile. Resident warps: 16 per SM (2,368).
+// Work items per tile list (log2) by the number of lists. A list is one warp's work, about 3 us per tile. Resident warps: 16 per SM (2,368).
 // With fewer than about seven lists per warp the launch ends with most warps
 // idle behind the longest lists, so lists are split; splitting costs a list's
 // set-up per part, so large systems keep one part.
-int splitOf(const nbk_context* h, int key) {
-  if (h->tuneSplitLog2[key] >= 0) return h->tuneSplitLog2[key];
+int splitRule(const nbk_context* h) {
   const int warps = 16 * h->numSM;
   return h->numLists >= 7 * warps ? 0 : h->numLists >= 3 * warps ? 1 : 2;
+}
+
+// The same unless the tuner or the caller chose.
+int splitOf(const nbk_context* h, int key) {
+  return h->tuneSplitLog2[key] >= 0 ? h->tuneSplitLog2[key] : splitRule(h);
 }
 
 // The slow-term tables reach pairlistdist^2 + 2, but a caller may build its lists
@@ -1015,7 +1018,10 @@ NBK_API int nbk_adjoint(nbk_handle h, unsigned flags, const nbk_float4* d_wF, co
   a.stride = n;
   a.gradAB = d_gradAB;
   a.gradCopies = h->adjAB.p;
-  a.splitLog2 = splitOf(h, tuneKey(h, NBK_ENERGY | flags));
+  // not the tuner's choice: the i sums are FP32 over a list part, so their bits
+  // follow the parts (whole groups of four tiles, as in the force kernel, make the
+  // parts uneven: 151 -> 160 us at 24,000 atoms; groups of two 158 us)
+  a.splitLog2 = splitRule(h);
   a.workCounter = h->counters.p + 2;
   NBK_CUDA(timedEvent(h, kTimedStart, st), "timing event");
   NBK_CUDA(launchAdjoint(a, slow, h->numSM, n, reinterpret_cast<float4*>(d_gradXQ), st), "adjoint kernel");

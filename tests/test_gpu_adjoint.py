@@ -62,3 +62,29 @@ def test_lj_parameter_gradients(case):
     sol = slice(0, dim - 2)
     print(f"sigma grad rms rel {rms_rel(gs[sol], rs[sol]):.2e}, eps {rms_rel(ge[sol], re_[sol]):.2e}")
     assert rms_rel(gs[sol], rs[sol]) <= 1e-4 and rms_rel(ge[sol], re_[sol]) <= 1e-4
+
+
+@pytest.mark.parametrize("slow", [True, False])
+def test_gradients_do_not_depend_on_the_launch_shape(slow):
+    """The fixed-point gradients are the same bits whatever launch shape the tuner
+    or the caller chose for the force kernel."""
+    import torch
+    s = mixed_box(seed=35, natoms=9001)
+    p = nbk.Packed(s)
+    n, dim = p.atomStorageSize, s.lj_table()[0]
+    nb = nbk.Nonbonded(PARAMS, s.lj_table())
+    nb.setup(p)
+    nb.build_tile_lists(p)
+    nb.force(p, ALL | nbk.NBK_PAIRLIST, xyzq=p.xyzq)
+    rng = np.random.default_rng(3)
+    w = torch.from_numpy(rng.standard_normal((n, 4)).astype(np.float32)).cuda()
+    g = torch.zeros((n, 4), device="cuda")
+    fixed = torch.zeros((4, n), dtype=torch.int64, device="cuda")
+    gab = torch.zeros(2 * dim * dim, dtype=torch.float64, device="cuda")
+    got = []
+    for split in (1, 2, 4):
+        nb.set_tuning(nbk.NBK_ENERGY | (nbk.NBK_SLOW if slow else 0), 4, split)
+        nb.adjoint(w, w, 0.1, 0.1, 0.1, g, gab, grad_fixed=fixed, slow=slow)
+        got.append((fixed.cpu().numpy(), g.cpu().numpy()))
+    for f, x in got[1:]:
+        assert np.array_equal(f, got[0][0]) and np.array_equal(x, got[0][1])
