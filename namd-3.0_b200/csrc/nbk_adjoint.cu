@@ -227,23 +227,21 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
             rad = fma2(mul2(pS, f2(4.0f)), mul2(qq, d2s), rad);
             qr = fma2(f2(a.cS), gs, qr);
             dqq = fma2(pS, gs, fma2(f2(a.cS), phis, dqq));
-            float2 gq = mul2(qq, gs);
-            gq = make_float2(aA ? gq.x : 0.f, aB ? gq.y : 0.f);
-            VX = fma2(gq, WX, make_float2(aA ? VX.x : 0.f, aB ? VX.y : 0.f));
-            VY = fma2(gq, WY, make_float2(aA ? VY.x : 0.f, aB ? VY.y : 0.f));
-            VZ = fma2(gq, WZ, make_float2(aA ? VZ.x : 0.f, aB ? VZ.y : 0.f));
-          } else {
-            VX = make_float2(aA ? VX.x : 0.f, aB ? VX.y : 0.f);
-            VY = make_float2(aA ? VY.x : 0.f, aB ? VY.y : 0.f);
-            VZ = make_float2(aA ? VZ.x : 0.f, aB ? VZ.y : 0.f);
+            const float2 gq = mul2(qq, gs);
+            VX = fma2(gq, WX, VX);
+            VY = fma2(gq, WY, VY);
+            VZ = fma2(gq, WZ, VZ);
           }
           rad = fma2(qq, qr, rad);
-          // an element that is no interacting pair may hold anything: exact zeros
-          rad = make_float2(aA ? rad.x : 0.f, aB ? rad.y : 0.f);
-          dqq = make_float2(aA ? dqq.x : 0.f, aB ? dqq.y : 0.f);
           VX = fma2(rad, DX, VX);
           VY = fma2(rad, DY, VY);
           VZ = fma2(rad, DZ, VZ);
+          // an element that is no interacting pair may hold anything (a padding
+          // slot's cotangent may be NaN): exact zeros in place of what it adds
+          VX = make_float2(aA ? VX.x : 0.f, aB ? VX.y : 0.f);
+          VY = make_float2(aA ? VY.x : 0.f, aB ? VY.y : 0.f);
+          VZ = make_float2(aA ? VZ.x : 0.f, aB ? VZ.y : 0.f);
+          dqq = make_float2(aA ? dqq.x : 0.f, aB ? dqq.y : 0.f);
           gi[I][0] += VX.x + VX.y;
           gi[I][1] += VY.x + VY.y;
           gi[I][2] += VZ.x + VZ.y;

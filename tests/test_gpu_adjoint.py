@@ -88,3 +88,45 @@ def test_gradients_do_not_depend_on_the_launch_shape(slow):
         got.append((fixed.cpu().numpy(), g.cpu().numpy()))
     for f, x in got[1:]:
         assert np.array_equal(f, got[0][0]) and np.array_equal(x, got[0][1])
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_cotangents_of_padding_slots_are_not_used(bad):
+    """No pair holds a padding slot, so whatever stands there changes no bit; and
+    a real atom's cotangent reaches its interacting partners only."""
+    import torch
+    s = mixed_box(seed=36, natoms=6001)
+    p = nbk.Packed(s)
+    n, dim = p.atomStorageSize, s.lj_table()[0]
+    real = real_slots(p)
+    assert (~real).sum() > 0
+    nb = nbk.Nonbonded(PARAMS, s.lj_table())
+    nb.setup(p)
+    nb.build_tile_lists(p)
+    nb.force(p, ALL | nbk.NBK_PAIRLIST, xyzq=p.xyzq)
+    rng = np.random.default_rng(3)
+    w = rng.standard_normal((n, 4)).astype(np.float32)
+    gab = torch.zeros(2 * dim * dim, dtype=torch.float64, device="cuda")
+
+    def grad(wF, wS):
+        g = torch.zeros((n, 4), device="cuda")
+        fixed = torch.zeros((4, n), dtype=torch.int64, device="cuda")
+        nb.adjoint(torch.from_numpy(wF).cuda(), torch.from_numpy(wS).cuda(), 0.1, 0.1, 0.1, g, gab,
+                   grad_fixed=fixed)
+        return fixed.cpu().numpy()
+
+    want = grad(w, w)
+    padded = w.copy()
+    padded[~real] = bad
+    assert np.array_equal(grad(padded, padded), want)
+    # one real atom with a bad cotangent: atoms further from it than the cutoff
+    # (minimum image, by 0.1 A) keep their bits
+    slot = p.slotOfAtom
+    one = w.copy()
+    one[slot[0]] = bad
+    box = s.arrays()["box"]
+    d = s.arrays()["pos"] - s.arrays()["pos"][0]
+    d -= box * np.rint(d / box)
+    far = slot[(d ** 2).sum(1) > (PARAMS.cutoff + 0.1) ** 2]
+    assert len(far) > 100
+    assert np.array_equal(grad(one, one)[:, far], want[:, far])
