@@ -1309,26 +1309,29 @@ NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* str
     return setErr(NBK_ERR_CUDA, "nbk_autotune: event");
   }
   // shapes are timed back to back on a warm L2; another shape replaces the
-  // default (kDefaultMinBlocks CTAs per SM, splitOf's warps per list) only when it is
-  // at least 3% faster, so that timing noise does not pick a shape that loses
-  // in use
+  // default (kDefaultMinBlocks CTAs per SM, splitRule's warps per list) only when it
+  // is at least 3% faster, so that timing noise does not pick a shape that loses
+  // in use. A default that is kept stays the rule, for whatever lists come next.
   float bestMs = 1e30f, defaultMs = 1e30f;
-  h->tuneSplitLog2[key] = -1;
-  const int defaultS = splitOf(h, key);
+  const int defaultS = splitRule(h);
   int bestB = kDefaultMinBlocks, bestS = defaultS;
   cudaError_t err = cudaSuccess;
   const int shapes[3] = {4, 5, 6};
   for (int bi = 0; bi < 3 && err == cudaSuccess; ++bi) {
     for (int sl = 0; sl <= maxSplitLog2 && err == cudaSuccess; ++sl) {
       a.splitLog2 = sl;
+      ForceArgs pa = a;
+      pa.workCounter = h->counters.p + 4;
       for (int it = -1; it < iterations && err == cudaSuccess; ++it) {  // it = -1: untimed
         if (it == 0) err = cudaEventRecord(e0, st);
         if (err == cudaSuccess) err = cudaMemsetAsync(h->force.p, 0, sizeof(long long) * 6 * (size_t)n, st);
         if (err == cudaSuccess)
           err = cudaMemsetAsync(h->acc.p, 0, sizeof(long long) * kAccCount * (size_t)accBlocks, st);
-        if (err == cudaSuccess) err = cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int), st);
+        if (err == cudaSuccess) err = cudaMemsetAsync(h->counters.p + 2, 0, sizeof(int) * 3, st);
         if (err == cudaSuccess) err = launchForce(a, kflags, shapes[bi], h->numSM, st);
-        h->launches += 1;
+        // the parts hold for the precise kernel too
+        if (err == cudaSuccess) err = launchPrecise(pa, kflags, h->numSM, st);
+        h->launches += needsPrecise(kflags) ? 2 : 1;
       }
       if (err == cudaSuccess) err = cudaEventRecord(e1, st);
       if (err == cudaSuccess) err = cudaEventSynchronize(e1);
@@ -1350,7 +1353,7 @@ NBK_API int nbk_autotune(nbk_handle h, unsigned flags, int iterations, void* str
   if (err != cudaSuccess) return setErr(NBK_ERR_CUDA, std::string("nbk_autotune: ") + cudaGetErrorString(err));
   if (!(bestMs < 0.97f * defaultMs)) {
     bestB = kDefaultMinBlocks;
-    bestS = defaultS;
+    bestS = -1;
     bestMs = defaultMs;
   }
   h->tuneMinBlocks[key] = bestB;

@@ -593,7 +593,7 @@ class Nonbonded:
                 "nbk_set_tuning")
 
     def tuning(self, flags=NBK_ENERGY | NBK_VIRIAL | NBK_SLOW):
-        """(CTAs per SM, warps per tile list, ms per force launch) for these flags."""
+        """(CTAs per SM, warps per tile list, ms per evaluation of the kernels) for these flags."""
         b, sp, ms = C.c_int(0), C.c_int(0), C.c_float(0)
         _dcheck(dev_lib().nbk_get_tuning(self._h, flags, C.byref(b), C.byref(sp), C.byref(ms)),
                 "nbk_get_tuning")
