@@ -48,14 +48,21 @@ __device__ __forceinline__ int splitPoint(int begin, int end) {
   return split;
 }
 
+// A coordinate as an integer of the same order, -0 as 0. NaN, which no comparison
+// of doubles orders, lies beyond the infinities.
+__device__ __forceinline__ long long orderKey(const double v) {
+  const long long b = __double_as_longlong(v + 0.0);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
 // One block per patch, a thread per position (more positions than threads go
 // round). Shared memory (dynamic) per atom for maxN atoms: x, y, z and the
 // current split key (double), id, ord, tmp, the position's part and its rank (int).
 //
 // Every level orders all parts at once: a thread counts the keys of its
 // position's part that are below its own, one FP64 compare a candidate read as
-// a broadcast, and equal keys are found afterwards, as two atoms with one rank,
-// and only then told apart by id. What bounds it is the sum of those counts,
+// a broadcast, and equal keys (and NaN) are found afterwards, as two atoms with
+// one rank, and only then told apart by id. What bounds it is the sum of those counts,
 // about 2 n^2 compares a patch over the levels, and the barriers between the
 // steps. 92,224 atoms in 320 patches: 188 us when the parts of a level were
 // taken one after the other by the whole block.
@@ -195,7 +202,9 @@ __global__ void __launch_bounds__(kSortMaxThreads)
       }
       __syncthreads();
       // an atom that does not find itself at its rank shares its coordinate
-      // with another: its rank is taken again below, with the id as tie break
+      // with another (or one of them is NaN): ranks are taken again below, with
+      // the id as tie break. Otherwise the ranks fill every part; where they did
+      // not, the order would hold what the shared memory did before.
       for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const int r = s_part[k];
         if (r < 0 || s_rs[r] < 0) continue;
@@ -215,8 +224,33 @@ __global__ void __launch_bounds__(kSortMaxThreads)
             rank += (kc < ka || (kc == ka && s_id[s_ord[m]] < ia)) ? 1 : 0;
           }
           s_tmp[b + rank] = s_ord[k];
+          s_rank[k] = b + rank;
         }
         __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+          const int r = s_part[k];
+          if (r < 0 || s_rs[r] < 0) continue;
+          if (s_tmp[s_rank[k]] != s_ord[k]) s_tie = 2;
+        }
+        __syncthreads();
+        if (s_tie == 2) {  // block-uniform: NaN, or two atoms with one id
+          // a strict order of any input: by coordinate, id and position
+          for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            const int r = s_part[k];
+            if (r < 0 || s_rs[r] < 0) continue;
+            const int b = rb[r], e = re[r];
+            const long long ka = orderKey(s_key[k]);
+            const int ia = s_id[s_ord[k]];
+            int rank = 0;
+            for (int m = b; m < e; ++m) {
+              const long long kc = orderKey(s_key[m]);
+              const int ic = s_id[s_ord[m]];
+              rank += (kc < ka || (kc == ka && (ic < ia || (ic == ia && m < k)))) ? 1 : 0;
+            }
+            s_tmp[b + rank] = s_ord[k];
+          }
+          __syncthreads();
+        }
       }
       for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const int r = s_part[k];

@@ -137,3 +137,43 @@ def test_patch_sort_order_with_equal_coordinates(grid):
     for q in range(L.numPatches):
         b, k = L.records[q, 1], L.records[q, 3]
         assert np.array_equal(got[b:b + k], _bisect(pos[b:b + k], L.ids[b:b + k])), q
+
+
+# Whatever the coordinates and ids hold (a blown-up integration, NaN or infinities
+# among them), the order of a patch is a permutation of its atoms; patches without
+# such atoms keep their order, and signed zeros are equal.
+@pytest.mark.parametrize("bad", ["one nan", "all nan", "inf", "same ids", "zeros"])
+def test_patch_sort_orders_any_input(bad):
+    import torch
+    s = mixed_box(seed=9, natoms=5003)
+    L = nbk.ResidentLayout(s, nbk.Packed(s), shuffle_seed=3)
+    pos, ids = L.pos.T.copy(), L.ids.copy()
+    hit = range(0, L.numPatches, 2)
+    rng = np.random.default_rng(1)
+    for q in hit:
+        b, k = L.records[q, 1], L.records[q, 3]
+        part = pos[b:b + k]
+        if bad == "one nan":
+            part[k // 2] = np.nan
+        elif bad == "all nan":
+            part[:] = np.nan
+        elif bad == "inf":
+            part[rng.random(part.shape) < 0.3] = np.inf
+            part[rng.random(part.shape) < 0.3] = -np.inf
+            part[rng.random(part.shape) < 0.1] = np.nan
+        elif bad == "same ids":
+            ids[b:b + k] = 7
+            part[:] = np.round(part / 4.0) * 4.0
+        else:
+            part[:] = rng.choice([0.0, -0.0, 1.0], part.shape)
+    for k, axis in enumerate("xyz"):
+        L.dev[axis] = torch.from_numpy(np.ascontiguousarray(pos[:, k])).cuda()
+    L.dev["id"] = torch.from_numpy(ids).cuda()
+    order = torch.zeros(len(ids), dtype=torch.int32, device="cuda")
+    L.sort_patch_atoms(order)
+    got = order.cpu().numpy()
+    for q in range(L.numPatches):
+        b, k = L.records[q, 1], L.records[q, 3]
+        assert np.array_equal(np.sort(got[b:b + k]), np.arange(k)), q
+        if q not in hit or bad == "zeros":
+            assert np.array_equal(got[b:b + k], _bisect(pos[b:b + k], ids[b:b + k])), q
