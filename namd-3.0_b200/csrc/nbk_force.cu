@@ -122,7 +122,8 @@ struct LaneSums {
 // interleaved copies in shared memory (s_slowTab), 16-byte pair n of row k of
 // copy c at s_slowTab[(k * P + n) * kCopies + c] with P = kSlowTableDeg1 / 2;
 // lane l reads copy l % kCopies, so with 8 copies the 8 lanes of a quarter
-// warp (one 16-byte bank group each) never conflict, whatever rows they read.
+// warp (one 16-byte bank group each) never conflict, whatever rows they read;
+// fewer copies conflict, at less than reads from the L1 cache cost.
 // kCopies == 0: the global copy (kSlowTableRow doubles per row); kBeyond: the
 // same, with pairs beyond the table from the formula.
 constexpr int kBeyond = -1;
@@ -927,15 +928,26 @@ static cudaError_t launchPC(const ForceArgs& a, int numSM, cudaStream_t st) {
                           a);
 }
 
-// the table in shared memory with 8 interleaved copies when they fit in 40 KB
-// (106 rows), else read from global memory; beyond its reach the instance that
-// can go on from there
+// The table in shared memory, in as many interleaved copies of 8, 4 or 1 as fit in
+// 40 KB (106, 213, 853 rows), else in global memory; beyond its reach the
+// instance that can go on from there. Global memory is the last choice because
+// what is left of the L1 cache for it follows the force kernel's shared memory:
+// while other kernels keep the SM busy the division stays. Energies, virials and
+// slow forces of 92,224 atoms with 739 rows: 528 us with 34 LJ types and 603 with
+// 61, which fill the SM's shared memory; with one copy here 519 and 525 (136
+// rows, four copies: 356 and 365 -> 343 and 347).
 template <bool E, bool V, bool S, bool B>
 static cudaError_t launchP(const ForceArgs& a, int numSM, cudaStream_t st) {
-  if (S && a.beyondTables) return launchPC<E, V, S, B, S ? kBeyond : 0>(a, numSM, st);
-  if (sizeof(double) * kSlowTableDeg1 * (size_t)a.slowTableRows * 8 <= 40 * 1024)
-    return launchPC<E, V, S, B, 8>(a, numSM, st);
-  return launchPC<E, V, S, B, 0>(a, numSM, st);
+  if constexpr (!S) {
+    return launchPC<E, V, S, B, 0>(a, numSM, st);
+  } else {
+    if (a.beyondTables) return launchPC<E, V, S, B, kBeyond>(a, numSM, st);
+    const size_t one = sizeof(double) * kSlowTableDeg1 * (size_t)a.slowTableRows, most = 40 * 1024;
+    if (8 * one <= most) return launchPC<E, V, S, B, 8>(a, numSM, st);
+    if (4 * one <= most) return launchPC<E, V, S, B, 4>(a, numSM, st);
+    if (one <= most) return launchPC<E, V, S, B, 1>(a, numSM, st);
+    return launchPC<E, V, S, B, 0>(a, numSM, st);
+  }
 }
 
 cudaError_t launchPrecise(const ForceArgs& a, unsigned flags, int numSM, cudaStream_t st) {

@@ -9,7 +9,8 @@ import pytest
 
 import nbk
 import oracle
-from helpers import ALL, FORCE_RMS_TOL, PARAMS, GpuRun, mixed_box, real_slots, rms_rel, water_box
+from helpers import (ALL, ENERGY_TOL, FORCE_RMS_TOL, PARAMS, VIRIAL_TOL, GpuRun, mixed_box, real_slots,
+                     rel, rms_rel, water_box)
 
 pytestmark = pytest.mark.gpu
 
@@ -88,6 +89,25 @@ def test_adjoint_table_placement(beta, pl, slow):
     ab = gab.cpu().numpy()
     assert rms_rel(ab[:dim * dim], gA.reshape(-1)) < FORCE_RMS_TOL
     assert rms_rel(ab[dim * dim:], gB.reshape(-1)) < FORCE_RMS_TOL
+
+
+# The precise kernel's table: eight, four copies or one in shared memory (40 KB), or
+# in global memory. Energies, slow virial and pair count as in every parity test.
+@pytest.mark.parametrize("beta,cutoff,pl,copies", [(0.2579, 12.0, 13.5, 8), (0.34, 10.0, 11.5, 4),
+                                                   (0.45, 9.0, 10.5, 1), (0.6, 12.0, 13.5, 1),
+                                                   (1.0, 12.0, 16.0, 0)])
+def test_precise_table_placement(beta, cutoff, pl, copies):
+    rows = nbk.slow_table(beta, cutoff, pl)[0].shape[0]
+    assert copies == next((c for c in (8, 4, 1) if rows * 48 * c <= 40 * 1024), 0)
+    params = dataclasses.replace(PARAMS, ewaldcof=beta, cutoff=cutoff, switchdist=cutoff - 1.0,
+                                 pairlistdist=pl)
+    p = nbk.Packed(mixed_box(seed=5, natoms=6200), patch_dim=pl)
+    run, (_, _, res, _) = _step(p, params, ALL)
+    _, _, ro = oracle.Oracle(p, params).forces(1)
+    for k in ("energyElec", "energySlow"):
+        assert rel(res[k], ro[k]) <= ENERGY_TOL, k
+    assert rms_rel(res["virialSlow"], ro["virialSlow"]) <= VIRIAL_TOL
+    assert run.nb.pair_count() == ro["pairs"]
 
 
 def _bisect(pos, ids):
