@@ -417,6 +417,11 @@ NBK_API int nbk_create(int deviceID, const nbk_params* p, nbk_handle* out) {
   h->pk.tabRows = buildForceTable(p->ewaldcof, p->cutoff, p->pairlistdist, ft, &ftStep);
   h->pk.tabStep = (float)ftStep;  // a power of two
   h->pk.tabInvStep = (float)(1.0 / ftStep);
+  if (rc == NBK_OK && h->pk.tabRows > 0) {
+    bool fits = true;
+    fin(forceTableFits(h->ljDim, h->pk.tabRows, &fits), "nbk_create: force table");
+    if (!fits) h->pk.tabRows = 0;  // the erfc form
+  }
   if (h->pk.tabRows > 0) {
     fin(h->forceTable.ensure(ft.size()), "nbk_create: alloc");
     if (rc == NBK_OK) fin(uploadNow(h->forceTable.p, ft.data(), sizeof(float4) * ft.size()), "nbk_create: copy");

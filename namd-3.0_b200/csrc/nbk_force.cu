@@ -23,6 +23,8 @@
 // FP64 geometry (see precisePass); its own
 // launch runs at higher occupancy than the register- and shared-memory-heavy
 // FP32 loop, which hides the FP64 dependency chains.
+#include <algorithm>
+
 #include "nbk_internal.cuh"
 #include "nbk_launch.h"
 
@@ -859,20 +861,45 @@ static cudaError_t launchT(const ForceArgs& a, int numSM, cudaStream_t st) {
   const size_t lj = B ? 0 : sizeof(float2) * (size_t)a.c.ljDim * a.c.ljDim;
   if constexpr (S) {
     if (a.pk.tabRows > 0 && !a.beyondTables) {  // the erfc form has no end
-      // as many copies of the table as fit in kForceTableBytes, up to the 8 that
-      // keep quarter warps free of bank conflicts
+      // copies of the table, up to the 8 that keep quarter warps free of bank
+      // conflicts, that cost no block: from 62 LJ types on the LJ table leaves no
+      // room for 8 beside four blocks, and a block counts for more (94 rows, fast
+      // and slow forces of 92,224 atoms: 70 types 287 -> 262 us, 80 types 371 ->
+      // 306, 110 types 622 -> 377)
       static KernelLimits limits;
       ForceArgs t = a;
       const size_t one = sizeof(float4) * (size_t)a.pk.tabRows;
-      t.tabCopies = 8;
-      while (t.tabCopies > 1 && one * t.tabCopies > kForceTableBytes) t.tabCopies /= 2;
-      return launchPersistent(forceKernel<E, V, S, true, B, MINB>, limits, kForceThreads,
-                              one * t.tabCopies + lj, numSM, st, t);
+      const auto kernel = forceKernel<E, V, S, true, B, MINB>;
+      int blocks = 0;
+      const cudaError_t e = limits.tableCopies(kernel, kForceThreads, lj, one, kForceTableBytes,
+                                               &t.tabCopies, &blocks);
+      if (e != cudaSuccess) return e;
+      return launchOverlapped(kernel, numSM * blocks, kForceThreads, one * t.tabCopies + lj, st, t);
     }
   }
   static KernelLimits limits;
   return launchPersistent(forceKernel<E, V, S, false, B, MINB>, limits, kForceThreads, lj, numSM,
                           st, a);
+}
+
+// A block less per SM costs more than the table gains over the erfc form: fast and
+// slow forces of 92,224 atoms with a table of 370 rows, 294 against 267 us with 70
+// LJ types (three blocks, four), 638 against 381 with 110 (one, two). One rule for
+// every flag combination and launch shape, and for replicas (whose LJ tables stay
+// in global memory), so that none of them changes a bit: by the shared memory of
+// the instance without energies at the default four blocks.
+cudaError_t forceTableFits(int ljDim, int rows, bool* fits) {
+  int dev = 0, perSM = 0, reserved = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&perSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+  cudaFuncAttributes at{};
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, forceKernel<false, false, true, true, false, 4>);
+  if (e != cudaSuccess) return e;
+  const size_t rest = at.sharedSizeBytes + (size_t)reserved + sizeof(float2) * (size_t)ljDim * ljDim;
+  auto blocks = [&](size_t bytes) { return std::min<size_t>((size_t)perSM / bytes, 4); };
+  *fits = blocks(rest + sizeof(float4) * (size_t)rows) == blocks(rest);
+  return cudaSuccess;
 }
 
 template <bool E, bool V, bool S, bool B>

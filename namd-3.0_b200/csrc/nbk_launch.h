@@ -47,9 +47,24 @@ class KernelLimits {
     d.next = (d.next + 1) % kSizes;
     return cudaSuccess;
   }
+  // Interleaved copies of a table of `one` bytes beside `rest` bytes of other dynamic
+  // shared memory: as many of 8, 4, 2, 1 as `most` bytes hold and as leave the
+  // blocks per SM that one copy leaves.
+  template <typename K>
+  cudaError_t tableCopies(K kernel, int threads, size_t rest, size_t one, size_t most, int* copies,
+                          int* blocks) {
+    cudaError_t e = blocksPerSM(kernel, threads, rest + one, blocks);
+    for (*copies = 8; e == cudaSuccess && *copies > 1; *copies /= 2) {
+      int nb = 0;
+      if (one * *copies > most) continue;
+      e = blocksPerSM(kernel, threads, rest + one * *copies, &nb);
+      if (nb == *blocks) break;
+    }
+    return e;
+  }
 
  private:
-  static constexpr int kDevices = 64, kSizes = 8;
+  static constexpr int kDevices = 64, kSizes = 16;
   struct PerDevice {
     size_t allowed = 0;
     size_t shmem[kSizes] = {};
@@ -117,6 +132,9 @@ int buildSlowTable(double beta, double cutoff, double pairlistdist, std::vector<
 // minBlocks: 4, 5 or 6 CTAs per SM (the register cap); a.splitLog2 set by the caller.
 cudaError_t launchForce(const ForceArgs& a, unsigned flags, int minBlocks, int numSM,
                         cudaStream_t st);
+// Whether the force kernel's slow table leaves it the blocks per SM that it has
+// without one.
+cudaError_t forceTableFits(int ljDim, int rows, bool* fits);
 // The precise energy / virial kernel after the force kernel (same lists, the
 // force kernel's live words, its own work counter a.workCounter); no-op when
 // flags need neither energies nor the slow virial.

@@ -10,7 +10,7 @@ import pytest
 import nbk
 import oracle
 from helpers import (ALL, ENERGY_TOL, FORCE_RMS_TOL, PARAMS, VIRIAL_TOL, GpuRun, mixed_box, real_slots,
-                     rel, rms_rel, water_box)
+                     rel, rms_rel, water_box, wider_lj)
 
 pytestmark = pytest.mark.gpu
 
@@ -89,6 +89,35 @@ def test_adjoint_table_placement(beta, pl, slow):
     ab = gab.cpu().numpy()
     assert rms_rel(ab[:dim * dim], gA.reshape(-1)) < FORCE_RMS_TOL
     assert rms_rel(ab[dim * dim:], gB.reshape(-1)) < FORCE_RMS_TOL
+
+
+# The LJ table in shared memory beside the slow table's copies: from 62 types on
+# fewer copies, and with many rows (the second coefficient) no table where one copy
+# costs a block. Types that no atom has change nothing but the form: with the
+# short table every bit stays; the erfc form holds the tolerance of every test.
+@pytest.mark.parametrize("beta,exact", [(0.2579, True), (0.6, False)])
+@pytest.mark.parametrize("types", [61, 62, 70, 80, 110])
+def test_wide_lj_tables(beta, exact, types):
+    params = dataclasses.replace(PARAMS, ewaldcof=beta)
+    p = nbk.Packed(mixed_box(seed=5, natoms=6200))
+    flags = ALL | nbk.NBK_CORRECTIONS
+    _, (F, S, res, X) = _step(p, params, flags)
+    run = GpuRun(p, params)
+    run.nb = nbk.Nonbonded(params, wider_lj(p.system.lj_table(), types))
+    run.nb.setup(p)
+    run.build()
+    run.eval(flags | nbk.NBK_PAIRLIST)
+    F1, S1, res1, X1 = run.eval(flags)
+    if exact:
+        assert np.array_equal(X, X1)
+        for k in res:
+            assert np.array_equal(res[k], res1[k]), k
+    assert rms_rel(F1, F) < FORCE_RMS_TOL and rms_rel(S1, S) < FORCE_RMS_TOL
+    # the launch shapes and the flags change no bit, whatever the form
+    for shape in ((4, 1), (5, 2), (6, 4)):
+        run.nb.set_tuning(flags, *shape)
+        assert np.array_equal(run.eval(flags)[3], X1)
+    assert np.array_equal(run.eval(nbk.NBK_SLOW | nbk.NBK_CORRECTIONS)[3], X1)
 
 
 # The precise kernel's table: eight, four copies or one in shared memory (40 KB), or
