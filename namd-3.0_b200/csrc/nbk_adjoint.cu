@@ -47,6 +47,10 @@ __device__ __forceinline__ SlowRow slowRow(const float4 a, const float4 b, const
 // memory with two reductions that nothing waits for. In shared memory an FP32
 // add is a compare-and-swap loop, and the water model's few types make lanes
 // meet in it: with one loop for both sums the kernel took 313 us.
+// Reductions of many blocks into one word follow one another: with sixteen tables
+// and all types wanted (the water model's pairs meet in a few words) 92,224 atoms
+// took 1,445 us, with sixty-four 559; 24,000 atoms with the solute's types alone
+// 151.5 and 148.8.
 template <bool doSlow, bool kShared>
 __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_constant__ AdjArgs a) {
   // the slow table's copies (kShared), the LJ table (A, -B)
@@ -290,13 +294,23 @@ __global__ void __launch_bounds__(kAdjThreads, 4) adjointKernel(const __grid_con
   }
 }
 
-// The LJ gradient tables' sum, copy by copy.
-__global__ void adjointTableKernel(int n, const double* __restrict__ copies, double* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// The LJ gradient tables' sum: a block sums 32 entries, each of its eight warps an
+// eighth of the copies.
+__global__ void __launch_bounds__(256) adjointTableKernel(int n, const double* __restrict__ copies,
+                                                          double* __restrict__ out) {
+  __shared__ double s_sum[8][32];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   double s = 0.0;
+  if (i < n) {
 #pragma unroll
-  for (int k = 0; k < kAdjCopies; ++k) s += copies[(size_t)k * n + i];
+    for (int k = 0; k < kAdjCopies / 8; ++k) s += copies[(size_t)(wib * (kAdjCopies / 8) + k) * n + i];
+  }
+  s_sum[wib][lane] = s;
+  __syncthreads();
+  if (wib || i >= n) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += s_sum[w][lane];
   out[i] = s;
 }
 
@@ -342,7 +356,7 @@ cudaError_t launchAdjoint(const AdjArgs& args, bool doSlow, int numSM, int n, fl
     e = launchAdj<true, false>(a, tables, numSM, st);
   }
   if (e != cudaSuccess) return e;
-  adjointTableKernel<<<(2 * d2 + 127) / 128, 128, 0, st>>>(2 * d2, a.gradCopies, a.gradAB);
+  adjointTableKernel<<<(2 * d2 + 31) / 32, 256, 0, st>>>(2 * d2, a.gradCopies, a.gradAB);
   e = cudaGetLastError();
   if (e != cudaSuccess || !out) return e;
   adjointOutKernel<<<min((n + 255) / 256, numSM * 4), 256, 0, st>>>(n, a.grad, a.stride, out);

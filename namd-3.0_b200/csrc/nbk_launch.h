@@ -221,7 +221,7 @@ void* mappedHostPointer(void* p);
 cudaError_t launchEnergyVirial(const long long* acc, nbk_virial_energy* out, cudaStream_t st,
                                int numReplicas = 1);
 
-constexpr int kAdjCopies = 16;
+constexpr int kAdjCopies = 64;  // a multiple of 8
 struct AdjArgs {
   const nbk_tile_list* lists;
   const int* numListsDev;
