@@ -18,7 +18,8 @@
 // reference accumulates FP32 atomics). One pass converts it to the FP32 grid
 // cuFFT transforms and clears it for the next step. Energies and virials are
 // reduced per block in FP64 and the block partials summed in a fixed order.
-// Each atom's force is one thread's sum in a fixed order.
+// Each atom's force is a sum in a fixed order (order 6 by one thread, orders 4 and 8
+// over lanes).
 #include <cuda_runtime.h>
 #include <cufft.h>
 
@@ -103,19 +104,37 @@ __device__ __forceinline__ void gridCell(const float4 a, int K1, int K2, int K3,
 // One warp spreads 32 atoms: each lane computes its atom's weights into
 // shared memory, then the warp walks the atoms, its lanes covering the
 // order^3 grid points of one atom (point p = lane + 32 h, x fastest, so
-// neighbouring lanes add to neighbouring addresses). Orders 4 and 6.
-template <int order>
+// neighbouring lanes add to neighbouring addresses). The weights lie in rows of 33
+// words, so that the lanes of a step, which read different k of one atom, read
+// from different banks (400,000 atoms at order 6 on a 1 A grid 224 -> 172 us; at
+// order 4 the same).
+//
+// kLarge (enough warps in flight that the atomics bound the kernel, not the latency
+// of the walk; orders 6 and 8): no atomic for a share that rounds to zero, as the
+// far corners of a high order's stencil do, and a warp takes eight groups of four
+// atoms from all over the array and walks them in turn, so that atoms which are
+// neighbours in space and in the array do not meet in one grid word one after the
+// other. Order 8, 92,224 atoms on a 1 A grid 92 -> 74 us, on a 2 A grid 104 -> 79,
+// 400,000 340 -> 275 and 364 -> 292; order 6 on a 1.5 A grid 54 -> 45 and 170 -> 163.
+// Below its sizes it loses (order 8, 3,000 atoms 20 -> 35 us; the sides meet near
+// 25,000 atoms, at order 6 near 45,000), and order 4 gains nothing. Two or three
+// near atoms in one step on the box that holds their stencils, the earlier form of
+// order 8, took 39, 81 and 339 us at 3,000, 92,224 and 400,000 atoms on a 2 A grid.
+template <int order, bool kLarge>
 __global__ void __launch_bounds__(128) spreadKernel(int n, const float4* __restrict__ atoms, int K1,
                                                     int K2, int K3,
                                                     unsigned long long* __restrict__ grid) {
   admitSuccessor();
   constexpr int kPts = order * order * order;
-  __shared__ float s_th[4][3][order][32];
+  __shared__ float s_th[4][3][order][33];
   __shared__ int s_i[4][3][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-  for (int a0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; a0 < n; a0 += warpsPerGrid * 32) {
-    const int i = a0 + lane;
+  const int K12 = K1 * K2;  // grid indices below 2^31 (checked at creation)
+  const int groups = (n + 31) >> 5;  // of 32 atoms
+  for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += warpsPerGrid) {
+    // at most 32 * groups - 1
+    const int i = kLarge ? 4 * (g + (lane >> 2) * groups) + (lane & 3) : 32 * g + lane;
     if (i < n) {
       const float4 at = atoms[i];
       int ix, iy, iz;
@@ -134,10 +153,12 @@ __global__ void __launch_bounds__(128) spreadKernel(int n, const float4* __restr
       s_i[wib][1][lane] = iy;
       s_i[wib][2][lane] = iz;
     }
+    const unsigned valid = kLarge ? __ballot_sync(0xffffffffu, i < n) : 0u;
     __syncwarp();
-    const int na = min(32, n - a0);
-    const int K12 = K1 * K2;  // grid indices below 2^31 (checked at creation)
-    for (int m = 0; m < na; ++m) {
+    const int walk = kLarge ? 32 : min(32, n - 32 * g);
+    for (int u = 0; u < walk; ++u) {
+      const int m = kLarge ? 4 * (u & 7) + (u >> 3) : u;  // the lane whose atom is next
+      if (kLarge && !((valid >> m) & 1u)) continue;       // warp-uniform
       const int bx = s_i[wib][0][m], by = s_i[wib][1][m], bz = s_i[wib][2][m];
 #pragma unroll
       for (int h = 0; h < (kPts + 31) / 32; ++h) {
@@ -152,131 +173,9 @@ __global__ void __launch_bounds__(128) spreadKernel(int n, const float4* __restr
           // v 2^32 is exact in FP32 (a power-of-two scaling), so this is the
           // same integer as the FP64 product rounded to the nearest
           const long long q = __float2ll_rn(v * kGridScale);
-          atomicAdd(&grid[x + K1 * y + K12 * z], (unsigned long long)q);
+          if (!kLarge || q) atomicAdd(&grid[x + K1 * y + K12 * z], (unsigned long long)q);
         }
       }
-    }
-    __syncwarp();
-  }
-}
-
-// Padded B-spline weights of a warp's 32 atoms, [axis][1 + k][atom], zero at
-// both ends. Rows of 33 words: the lanes of a step read different k of one
-// atom, in different banks.
-template <int order>
-using SpreadWeights = float[3][order + 2][33];
-
-// Adds the charges of `count` atoms of the warp, by lane: the lanes cover
-// the box of grid points that holds their stencils (point p = lane + 32 h, x
-// fastest, so neighbouring lanes add to neighbouring addresses). Each atom's
-// share of a point is rounded by itself, so the integers are the same however
-// the atoms are grouped.
-template <int order, int count>
-__device__ __forceinline__ void spreadGroup(const SpreadWeights<order>& th, const int4* cell,
-                                            const int (&m)[count], int lane, int K1, int K2, int K3,
-                                            unsigned long long* __restrict__ grid) {
-  constexpr int S = count > 1 ? order + 1 : order;  // the cells of a group differ by one at most
-  constexpr int kPts = S * S * S;
-  const int K12 = K1 * K2;  // grid indices below 2^31 (checked at creation)
-  int4 b = cell[m[0]];
-#pragma unroll
-  for (int c = 1; c < count; ++c) {
-    const int4 o = cell[m[c]];
-    b = make_int4(min(b.x, o.x), min(b.y, o.y), min(b.z, o.z), 0);
-  }
-  const float* t[3][count];
-#pragma unroll
-  for (int c = 0; c < count; ++c) {
-    const int4 o = cell[m[c]];
-    t[0][c] = &th[0][1 - (o.x - b.x)][m[c]];
-    t[1][c] = &th[1][1 - (o.y - b.y)][m[c]];
-    t[2][c] = &th[2][1 - (o.z - b.z)][m[c]];
-  }
-#pragma unroll
-  for (int h = 0; h < (kPts + 31) / 32; ++h) {
-    const int p = lane + 32 * h;
-    if (kPts % 32 == 0 || p < kPts) {
-      const int x0 = p % S, y0 = (p / S) % S, z0 = p / (S * S);
-      int x = b.x + x0, y = b.y + y0, z = b.z + z0;
-      if (x >= K1) x -= K1;
-      if (y >= K2) y -= K2;
-      if (z >= K3) z -= K3;
-      unsigned long long q = 0;
-#pragma unroll
-      for (int c = 0; c < count; ++c) {
-        const float v = t[0][c][33 * x0] * t[1][c][33 * y0] * t[2][c][33 * z0];
-        // v 2^32 is exact in FP32 (a power-of-two scaling), so this is the
-        // same integer as the FP64 product rounded to the nearest
-        q += (unsigned long long)__float2ll_rn(v * kGridScale);
-      }
-      if (q) atomicAdd(&grid[x + K1 * y + K12 * z], q);
-    }
-  }
-}
-
-// spreadKernel with two or three atoms in one step where their cells lie within
-// one of each other along every axis, so that a point they share gets one atomic:
-// in the order of the patches that leaves 47 of 64 points an atom at order 4 and a
-// 1 A grid, and fewer at the coarser grids of higher orders. Whole reciprocal
-// evaluation of 92k atoms: order 8 172 -> 138 us. Order 6 on a 1.5 A grid gains
-// nothing (105.1 and 105.3 us) and order 4 loses at 92k atoms (71.8 -> 73.9 us; 1.07M
-// atoms 528 -> 523): the longer box of a group costs them what the atomics save, so
-// they keep spreadKernel.
-template <int order>
-__global__ void __launch_bounds__(128) spreadGroupsKernel(int n, const float4* __restrict__ atoms,
-                                                          int K1, int K2, int K3,
-                                                          unsigned long long* __restrict__ grid) {
-  admitSuccessor();
-  __shared__ SpreadWeights<order> s_th[4];
-  __shared__ int4 s_cell[4][32];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) s_th[wib][d][0][lane] = s_th[wib][d][order + 1][lane] = 0.f;
-  for (int a0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; a0 < n; a0 += warpsPerGrid * 32) {
-    int4 cell = make_int4(0, 0, 0, 0);
-    bool finite = false;  // the padding gives no zero beside an infinity: such atoms go alone
-    if (a0 + lane < n) {
-      const float4 at = atoms[a0 + lane];
-      float w[3], t[order];
-      gridCell(at, K1, K2, K3, cell.x, cell.y, cell.z, w[0], w[1], w[2]);
-      finite = isfinite(at.w) && isfinite(w[0]) && isfinite(w[1]) && isfinite(w[2]);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        bsplineTheta<float, order>(w[d], t);
-#pragma unroll
-        for (int k = 0; k < order; ++k) s_th[wib][d][1 + k][lane] = d ? t[k] : at.w * t[k];
-      }
-    }
-    s_cell[wib][lane] = cell;
-    __syncwarp();
-    unsigned near = 0;  // the lanes whose cells lie within one of this lane's
-#pragma unroll 8
-    for (int j = 0; j < 32; ++j) {
-      const int4 o = s_cell[wib][j];
-      if (max(max(abs(o.x - cell.x), abs(o.y - cell.y)), abs(o.z - cell.z)) <= 1) near |= 1u << j;
-    }
-    const unsigned joins = __ballot_sync(0xffffffffu, finite);
-    near = finite ? near & joins : 0;
-    unsigned left = n - a0 < 32 ? (1u << (n - a0)) - 1 : ~0u;
-    while (left) {
-      const int first = __ffs(left) - 1;
-      left &= left - 1;
-      unsigned with = left & __shfl_sync(0xffffffffu, near, first);
-      if (!with) {
-        spreadGroup<order, 1>(s_th[wib], s_cell[wib], {first}, lane, K1, K2, K3, grid);
-        continue;
-      }
-      const int second = __ffs(with) - 1;
-      left ^= 1u << second;
-      with &= left & __shfl_sync(0xffffffffu, near, second);
-      if (!with) {
-        spreadGroup<order, 2>(s_th[wib], s_cell[wib], {first, second}, lane, K1, K2, K3, grid);
-        continue;
-      }
-      const int third = __ffs(with) - 1;
-      left ^= 1u << third;
-      spreadGroup<order, 3>(s_th[wib], s_cell[wib], {first, second, third}, lane, K1, K2, K3, grid);
     }
     __syncwarp();
   }
@@ -762,11 +661,12 @@ extern "C" NBK_API int nbk_pme_spread_charge(nbk_pme p, int n, const nbk_float4*
   if (n) {
     const int blocks = std::min((n + 127) / 128, p->numSM * 16);
     const float4* a = reinterpret_cast<const float4*>(atoms);
-    switch (p->order) {
-      case 4: spreadKernel<4><<<blocks, 128, 0, st>>>(n, a, p->K1, p->K2, p->K3, p->gridFixed); break;
-      case 6: spreadKernel<6><<<blocks, 128, 0, st>>>(n, a, p->K1, p->K2, p->K3, p->gridFixed); break;
-      default: spreadGroupsKernel<8><<<blocks, 128, 0, st>>>(n, a, p->K1, p->K2, p->K3, p->gridFixed); break;
-    }
+    // the sizes at which the large form begins, in warps per SM
+    const bool large = n >= (p->order == 6 ? 10 : 6) * 32 * p->numSM;
+    const auto kernel = p->order == 4   ? spreadKernel<4, false>
+                        : p->order == 6 ? (large ? spreadKernel<6, true> : spreadKernel<6, false>)
+                                        : (large ? spreadKernel<8, true> : spreadKernel<8, false>);
+    kernel<<<blocks, 128, 0, st>>>(n, a, p->K1, p->K2, p->K3, p->gridFixed);
     PME_CUDA(cudaGetLastError(), "nbk_pme_spread_charge");
   }
   PME_CUDA(launchOverlapped(gridToFloatKernel, (int)std::min<size_t>((ng + 255) / 256, (size_t)p->numSM * 8),

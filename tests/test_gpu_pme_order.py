@@ -13,12 +13,13 @@ pytestmark = pytest.mark.gpu
 
 # Sites far apart, each with atoms within one or two grid cells and some at the
 # ends of the box, site by site and dealt round the sites; one atom to 1,500, so
-# that the last warp of the gather is partly filled. The grid's integers are the
+# that the last warp of the gather is partly filled, and more than begin the large
+# form of the spread. The grid's integers are the
 # same, so energy, virial and each atom's force are equal bit for bit; energy and
 # virial hold the bounds of the PME tests.
 @pytest.mark.parametrize("order", [4, 6, 8])
 @pytest.mark.parametrize("n,K", [(1, (8, 8, 8)), (2, (16, 18, 20)), (3, (16, 18, 20)), (31, (8, 9, 10)),
-                                 (33, (32, 30, 36)), (1500, (64, 60, 72))])
+                                 (33, (32, 30, 36)), (1500, (64, 60, 72)), (60001, (64, 60, 72))])
 def test_pme_does_not_depend_on_the_atoms_order(order, n, K):
     rng = np.random.default_rng(100 * order + n)
     sites = rng.random((max(n // 3, 1), 3))
