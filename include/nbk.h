@@ -347,6 +347,13 @@ NBK_API const char* nbk_noalloc_last_error(void);
  * NBK_ERR_ARG for bad parameters. */
 NBK_API int nbk_slow_table(double ewaldcof, double cutoff, double pairlistdist, double* out,
                            int maxRows, double* step);
+/* The FP32 table of the slow force factor (dE/dr)/r that the force kernel evaluates
+ * over the same range, in the same layout with four floats per row (a cubic
+ * interpolant, within 3e-8 of the factor's largest value). Returns the number of
+ * rows, 0 when that takes more than 1,024: the kernel then forms the factor from
+ * erfc. Otherwise as nbk_slow_table. */
+NBK_API int nbk_force_table(double ewaldcof, double cutoff, double pairlistdist, float* out,
+                            int maxRows, double* step);
 
 /* ---- test hooks -------------------------------------------------------------- */
 

@@ -215,3 +215,17 @@ extern "C" NBK_API int nbk_slow_table(double ewaldcof, double cutoff, double pai
   }
   return rows;
 }
+
+extern "C" NBK_API int nbk_force_table(double ewaldcof, double cutoff, double pairlistdist,
+                                       float* out, int maxRows, double* step) {
+  if (!(cutoff > 0) || pairlistdist < cutoff || !(ewaldcof >= 0)) return NBK_ERR_ARG;
+  std::vector<float4> t;
+  double D = 0.0;
+  const int rows = nbk::buildForceTable(ewaldcof, cutoff, pairlistdist, t, &D);
+  if (step) *step = D;
+  if (out && rows > 0) {
+    if (maxRows < rows) return NBK_ERR_ARG;
+    std::memcpy(out, t.data(), sizeof(float4) * t.size());
+  }
+  return rows;
+}

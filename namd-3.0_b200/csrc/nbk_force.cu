@@ -883,7 +883,7 @@ static cudaError_t launchT(const ForceArgs& a, int numSM, cudaStream_t st) {
 }
 
 // A block less per SM costs more than the table gains over the erfc form: fast and
-// slow forces of 92,224 atoms with a table of 370 rows, 294 against 267 us with 70
+// slow forces of 92,224 atoms with a table of 739 rows, 294 against 267 us with 70
 // LJ types (three blocks, four), 638 against 381 with 110 (one, two). One rule for
 // every flag combination and launch shape, and for replicas (whose LJ tables stay
 // in global memory), so that none of them changes a bit: by the shared memory of

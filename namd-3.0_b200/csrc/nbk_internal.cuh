@@ -207,7 +207,7 @@ struct PackedConst {
 // The fit's error relative to the factor's largest value (at r = 0), and the
 // rows a table may have (16 KB of shared memory). At 3e-8 the fit is an order
 // below the rounding of the erfc form ((1 - erfc term) r^-3 cancels at short
-// range), and the benchmark's parameters give 93 rows.
+// range), and the benchmark's parameters give 94 rows.
 constexpr double kForceTableTol = 3e-8;
 constexpr int kForceTableMaxRows = 1024;
 

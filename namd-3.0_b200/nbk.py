@@ -362,6 +362,8 @@ def dev_lib() -> C.CDLL:
         lib.nbk_measure_fp64_peak.argtypes = [i, C.POINTER(C.c_double)]
         lib.nbk_debug_fail_alloc.argtypes = [i]
         lib.nbk_get_precise_times.argtypes = [vp, C.POINTER(C.c_float), i, C.POINTER(i)]
+        lib.nbk_force_table.argtypes = [C.c_double, C.c_double, C.c_double, vp, i,
+                                        C.POINTER(C.c_double)]
         lib.nbk_slow_table.argtypes = [C.c_double, C.c_double, C.c_double, vp, i,
                                        C.POINTER(C.c_double)]
         lib.nbk_set_replicas.argtypes = [vp, i, vp, vp, vp, vp, vp, vp, vp, vp]
@@ -663,6 +665,20 @@ def slow_table(ewaldcof: float, cutoff: float, pairlistdist: float):
     rc = L.nbk_slow_table(ewaldcof, cutoff, pairlistdist, out.ctypes.data, rows, C.byref(step))
     if rc != rows:
         raise NbkError(f"nbk_slow_table failed ({rc})")
+    return out, step.value
+
+
+def force_table(ewaldcof: float, cutoff: float, pairlistdist: float):
+    """The FP32 slow-force table of the force kernel (nbk_force_table): (rows, step),
+    four floats a row; no rows when the kernel takes the erfc form. Host-only."""
+    L = dev_lib()
+    step = C.c_double(0.0)
+    rows = L.nbk_force_table(ewaldcof, cutoff, pairlistdist, None, 0, C.byref(step))
+    if rows < 0:
+        raise NbkError(f"nbk_force_table failed ({rows})")
+    out = np.zeros((rows, 4), dtype=np.float32)
+    if rows and L.nbk_force_table(ewaldcof, cutoff, pairlistdist, out.ctypes.data, rows, None) != rows:
+        raise NbkError("nbk_force_table failed")
     return out, step.value
 
 

@@ -33,6 +33,15 @@ def wider_lj(lj, types):
     return tuple(out)
 
 
+def split_rule(packed):
+    """Warps per list of an untuned handle: by the number of lists and of SMs."""
+    import torch
+    tiles = (packed.patches[:, 0] + 31) // 32
+    lists = int(tiles[packed.computes_patch[:, 0]].sum())
+    warps = 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    return 1 if lists >= 7 * warps else 2 if lists >= 3 * warps else 4
+
+
 def rms_rel(a, b):
     num = np.sqrt(((a - b) ** 2).sum())
     den = np.sqrt((b ** 2).sum())

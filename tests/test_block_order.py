@@ -2,7 +2,10 @@
 atoms, lane l and bit 8 J + 4 e + I standing for the pair i = 8 I + (l & 7),
 j = 8 J + (4 e ^ (l & 4)) + (l >> 3). Restated here from the kernels' shuffles
 (blockOrder), the precise kernel's decoding of a live word's bit, and the
-export's way back to the interface's order (bit t of lane i <-> j = (i + t) & 31)."""
+export's way back to the interface's order (bit t of lane i <-> j = (i + t) & 31).
+This pins the arithmetic of the order; that the kernels follow it is what the
+pair-set tests check on a GPU, whose exported masks went through the order and
+back, and the force tests."""
 import numpy as np
 import pytest
 

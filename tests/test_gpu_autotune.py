@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import nbk
-from helpers import ALL, GpuRun, mixed_box
+from helpers import ALL, GpuRun, mixed_box, split_rule
 
 pytestmark = pytest.mark.gpu
 
@@ -59,20 +59,11 @@ def test_launch_sequence_per_register_cap():
         run.eval(ALL)
 
 
-def _rule(packed):
-    """Warps per list of an untuned handle: by the number of lists and of SMs."""
-    import torch
-    tiles = (packed.patches[:, 0] + 31) // 32
-    lists = int(tiles[packed.computes_patch[:, 0]].sum())
-    warps = 16 * torch.cuda.get_device_properties(0).multi_processor_count
-    return 1 if lists >= 7 * warps else 2 if lists >= 3 * warps else 4
-
-
 def test_a_tuner_that_keeps_the_default_keeps_the_rule():
     """A shape that does not beat the default leaves the rule on the number of
     lists in force: the same handle on another layout takes that layout's."""
     small, large = nbk.Packed(mixed_box(natoms=6000)), nbk.Packed(mixed_box(natoms=50003))
-    assert (_rule(small), _rule(large)) == (4, 1)
+    assert (split_rule(small), split_rule(large)) == (4, 1)
     run = GpuRun(large)
     run.build()
     run.eval(ALL | nbk.NBK_PAIRLIST)

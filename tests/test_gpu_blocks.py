@@ -10,7 +10,7 @@ import pytest
 import nbk
 import oracle
 from helpers import (ALL, ENERGY_TOL, FORCE_RMS_TOL, PARAMS, VIRIAL_TOL, GpuRun, mixed_box, real_slots,
-                     rel, rms_rel, water_box, wider_lj)
+                     rel, rms_rel, split_rule, water_box, wider_lj)
 
 pytestmark = pytest.mark.gpu
 
@@ -22,14 +22,16 @@ def _step(p, params, flags):
     return run, run.eval(flags)
 
 
-# A table has (pairlistdist^2 + 2) / step rows, the step falling with beta^2: 93
-# rows at the first parameters, one row of a step at the second, and more than
-# the table may have (1,024, at beta pairlistdist of about 12) at the last two,
-# which take the erfc form. Tolerance: that of every force test against FP64.
-@pytest.mark.parametrize("beta,cutoff,switch,pl", [(0.2579, 12.0, 10.0, 13.5), (0.02, 9.0, 7.0, 10.5),
-                                                   (0.6, 9.0, 9.0, 10.5), (1.0, 12.0, 10.0, 13.5),
-                                                   (1.2, 12.0, 10.0, 16.0)])
-def test_slow_force_table_and_erfc_form(beta, cutoff, switch, pl):
+# A table has (pairlistdist^2 + 2) / step rows, the step falling with beta^2: 94
+# rows at the first parameters (eight copies), six at the second, one copy at the
+# third, and more than the table may have (1,024, at beta pairlistdist of about 12)
+# at the last two, which take the erfc form. Tolerance: that of every force test
+# against FP64.
+@pytest.mark.parametrize("beta,cutoff,switch,pl,rows", [
+    (0.2579, 12.0, 10.0, 13.5, 94), (0.02, 9.0, 7.0, 10.5, 6), (0.6, 9.0, 9.0, 10.5, 451),
+    (0.6, 12.0, 10.0, 13.5, 739), (1.0, 12.0, 10.0, 13.5, 0), (1.2, 12.0, 10.0, 16.0, 0)])
+def test_slow_force_table_and_erfc_form(beta, cutoff, switch, pl, rows):
+    assert len(nbk.force_table(beta, cutoff, pl)[0]) == rows
     params = dataclasses.replace(PARAMS, ewaldcof=beta, cutoff=cutoff, switchdist=switch,
                                  pairlistdist=pl)
     p = nbk.Packed(mixed_box(seed=5, natoms=6200), patch_dim=pl)
@@ -41,30 +43,34 @@ def test_slow_force_table_and_erfc_form(beta, cutoff, switch, pl):
 
 
 # 1, 2 or 4 work items per list by the rule on their number: every sum is the
-# one of unsplit lists, bit for bit (the force and the precise kernel).
-@pytest.mark.parametrize("make", [lambda: water_box(seed=3, nwater=900, box=30.0),
-                                  lambda: mixed_box(seed=4, natoms=9001),
-                                  lambda: mixed_box(seed=4, natoms=24000),
-                                  lambda: mixed_box(seed=4, natoms=50003)])
-def test_split_lists_give_the_sums_of_whole_lists(make):
+# one of unsplit lists, bit for bit (the force and the precise kernel), and of the
+# other splits.
+@pytest.mark.parametrize("make,split", [(lambda: water_box(seed=3, nwater=900, box=30.0), 4),
+                                        (lambda: mixed_box(seed=4, natoms=9001), 4),
+                                        (lambda: mixed_box(seed=4, natoms=24000), 2),
+                                        (lambda: mixed_box(seed=4, natoms=50003), 1)])
+def test_split_lists_give_the_sums_of_whole_lists(make, split):
     p = nbk.Packed(make())
+    assert split_rule(p) == split
     run, (_, _, res, X) = _step(p, PARAMS, ALL)
-    split = run.nb.tuning(ALL)["warps_per_list"]
-    assert split in (1, 2, 4)
-    run.nb.set_tuning(ALL, 4, 1)
-    _, _, one, X1 = run.eval(ALL)
-    assert np.array_equal(X, X1)
-    for k in res:
-        assert np.array_equal(res[k], one[k]), k
+    assert run.nb.tuning(ALL)["warps_per_list"] == split
+    for other in {1, 2, 4} - {split}:
+        run.nb.set_tuning(ALL, 4, other)
+        _, _, one, X1 = run.eval(ALL)
+        assert np.array_equal(X, X1)
+        for k in res:
+            assert np.array_equal(res[k], one[k]), k
 
 
 # The adjoint's slow table: eight copies in shared memory; one copy at the small
 # steps of a large beta; global memory when not even one fits (more than 768
 # rows). Also without the slow term. Tolerance: FP32 pair terms, as the forces.
-@pytest.mark.parametrize("beta,pl,slow", [(0.2579, 13.5, True), (1.0, 13.5, True), (1.0, 16.0, True),
-                                          (0.2579, 13.5, False)])
-def test_adjoint_table_placement(beta, pl, slow):
+@pytest.mark.parametrize("beta,pl,slow,copies", [(0.2579, 13.5, True, 8), (1.0, 13.5, True, 1),
+                                                 (1.0, 16.0, True, 0), (0.2579, 13.5, False, 8)])
+def test_adjoint_table_placement(beta, pl, slow, copies):
     import torch
+    rows = len(nbk.slow_table(beta, PARAMS.cutoff, pl)[0])  # 32 bytes each in FP32, in 24 KB
+    assert copies == next((c for c in (8, 4, 2, 1) if rows * 32 * c <= 24 * 1024), 0)
     params = dataclasses.replace(PARAMS, ewaldcof=beta, pairlistdist=pl)
     sy = mixed_box(seed=6, natoms=6200)
     p = nbk.Packed(sy, patch_dim=pl)

@@ -61,3 +61,38 @@ def test_slow_table_rejects_bad_parameters():
     rows = L.nbk_slow_table(0.26, 12.0, 13.5, None, 0, None)
     out = np.zeros((rows - 1, DEG + 1))
     assert L.nbk_slow_table(0.26, 12.0, 13.5, out.ctypes.data, rows - 1, None) < 0
+
+
+# The force kernel's cubic FP32 table: 94 rows at the benchmark's parameters, few for
+# a small Ewald coefficient, many for a large one, none where 1,024 are not enough.
+@pytest.mark.parametrize("beta,cutoff,pl,rows", [(0.2579, 12.0, 13.5, 94), (0.02, 9.0, 10.5, 6),
+                                                 (0.34, 10.0, 11.5, 136), (0.6, 9.0, 10.5, 451),
+                                                 (1.0, 12.0, 13.5, 0), (1.2, 12.0, 16.0, 0)])
+def test_force_table_matches_the_slow_force_factor(beta, cutoff, pl, rows):
+    T, step = nbk.force_table(beta, cutoff, pl)
+    assert T.shape == (rows, 4)
+    if not rows:
+        return
+    assert step <= 32.0 and math.log2(step) == round(math.log2(step))
+    assert step * (rows - 1) + step / 2 >= pl * pl + 2
+    s = np.linspace(1.0, pl * pl, 200001)
+    r = np.sqrt(s)
+    g = (-1.0 / cutoff ** 3 + erf(beta * r) / r ** 3
+         - 2.0 * beta / math.sqrt(math.pi) * np.exp(-beta * beta * s) / s)
+    k = np.rint(s / step).astype(int)
+    w = s - step * k
+    c = T.astype(np.float64)[k]
+    got = ((c[:, 3] * w + c[:, 2]) * w + c[:, 1]) * w + c[:, 0]
+    # the builder's bound, 3e-8 of the factor at r = 0 plus 1/rc^3, and the rounding
+    # of the constant coefficient to FP32 (the others are smaller)
+    most = 4.0 * beta ** 3 / (3.0 * math.sqrt(math.pi))
+    bound = 3e-8 * (abs(most - cutoff ** -3) + cutoff ** -3) + 2.0 ** -24 * np.abs(g).max()
+    assert np.abs(got - g).max() <= 1.5 * bound
+
+
+def test_force_table_rejects_bad_parameters():
+    L = nbk.dev_lib()
+    assert L.nbk_force_table(0.26, -1.0, 13.5, None, 0, None) < 0
+    assert L.nbk_force_table(0.26, 12.0, 11.0, None, 0, None) < 0
+    out = np.zeros((93, 4), np.float32)
+    assert L.nbk_force_table(0.2579, 12.0, 13.5, out.ctypes.data, 93, None) < 0
