@@ -185,9 +185,9 @@ struct nbk_context {
 
 namespace {
 // Default launch shape of the force kernel: 4 CTAs per SM (a 128-register
-// cap), one warp per tile list; measured fastest at 92k atoms for the energy
-// and slow-force evaluations (steady steps, fast + slow forces 280 us against
-// 281 at 5 and 290 at 6 CTAs per SM; with energies and virials 494, 502, 510).
+// cap); measured fastest at 92k atoms (steady steps at 4, 5 and 6 CTAs per SM: fast
+// forces 177, 183, 195 us, fast + slow 250, 276, 293, with energies and virials 462,
+// 494, 522).
 constexpr int kDefaultMinBlocks = 4;
 constexpr int kMaxTimed = 4096;
 

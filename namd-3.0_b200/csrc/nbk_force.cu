@@ -9,8 +9,8 @@
 //     forces ride in registers and are reduced over lanes per row of blocks
 //     and per group of tiles;
 //   - blocks without listed pairs are skipped warp-uniformly;
-//   - the lists it reads are already refined (TileExcl masks from
-//     refineKernel, in block order); a pairlist step refines, compacts, then runs this kernel;
+//   - the lists it reads are already refined (masks from refineKernel, in block
+//     order); a pairlist step refines, puts the lists in order, then runs this kernel;
 //   - per-tile FP32 partial forces are folded into 64-bit fixed point with
 //     integer atomics, so the summed forces do not depend on the order in
 //     which lists run; the LJ energy is summed in FP32 per group of tiles and
@@ -393,9 +393,11 @@ __device__ __forceinline__ void reduceGroup(const int lane, LaneSums& L, long lo
 // passes) where the diagonals j = (l + t) & 31 of the tile held 17.4
 // (419,488), and the diagonals' rotation of the j sums (12 shuffles a pass)
 // becomes one reduction per row of blocks. Steady steps of the 92,224-atom
-// mixed system: fast + slow forces 392 -> 290 us, fast forces 279 -> 198 us,
-// with energies and virials 601 -> 507 us (of which the precise kernel is 200);
-// 210 M warp instructions for fast + slow forces.
+// mixed system, by diagonals, when the blocks came, and now (the slow table, i rows
+// kept once, overlapped launches): fast + slow forces 392, 290, 267 us, fast forces
+// 279, 198, 184, with energies and virials 601, 507, 483 (of which the precise
+// kernel is 197); 210 M warp instructions for fast + slow forces when the blocks
+// came, 195 M now.
 //
 // MINB: CTAs per SM the register budget is cut for (4, 5 or 6 -> 128, 96 or
 // 80 registers); a.splitLog2: each list's j tiles are shared by 2^splitLog2

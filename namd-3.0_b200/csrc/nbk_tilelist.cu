@@ -1,11 +1,11 @@
 // Tile-list build of the B200 nonbonded path: tile bounding boxes, bbox
-// culling of every (compute, i-tile) into a j-tile list, and the compaction
-// that follows the pairlist refinement.
+// culling of every (compute, i-tile) into a j-tile list, the pairlist refinement,
+// the order of the lists that it leaves, and the export.
 //
 // The reference (src/CudaTileListKernel.cu:1022-1192) culls with one thread
 // per i-tile looping over the partner patch's tiles, allocates output with
 // atomics and re-launches after a host synchronisation when its buffer
-// overflows. Here one warp culls one i-tile (its lanes test 32 j-tiles at a
+// overflows. Here half a warp culls one i-tile (its lanes test 16 j-tiles at a
 // time, ballot + popc place the survivors), and every list writes into a
 // slot range reserved on the host from the patch sizes, so the build never
 // overflows, never synchronises with the host and can be captured in a graph.
@@ -123,9 +123,9 @@ __global__ void buildListsKernel(int numLists, const ListSeed* __restrict__ seed
 }
 
 // After the pairlist refinement: the lists that kept tiles, in their order
-// (batched replicas, whose lists stay grouped by replica). A block of
-// kCompactWarps warps takes as many lists at a time as it has threads; one
-// thread reserves the output of all of them with one atomic on counters[0].
+// (batched replicas, whose lists stay grouped by replica). A block takes as many
+// lists at a time as it has threads; one thread reserves the output of all of them
+// with one atomic on counters[0].
 constexpr int kCompactThreads = 256;
 
 __global__ void __launch_bounds__(kCompactThreads)
