@@ -237,10 +237,11 @@ int tuneKey(const nbk_context* h, unsigned flags) {
          ((flags & NBK_SLOW) ? 1 : 0);
 }
 
-// Work items per tile list (log2) by the number of lists. A list is one warp's work, about 3 us per tile. Resident warps: 16 per SM (2,368).
-// With fewer than about seven lists per warp the launch ends with most warps
-// idle behind the longest lists, so lists are split; splitting costs a list's
-// set-up per part, so large systems keep one part.
+// Work items per tile list (log2) by the number of lists. A list is one warp's
+// work, about 3 us per tile. Resident warps: 16 per SM (2,368). With fewer than
+// about seven lists per warp the launch ends with most warps idle behind the longest
+// lists, so lists are split; splitting costs a list's set-up per part, so large
+// systems keep one part.
 int splitRule(const nbk_context* h) {
   const int warps = 16 * h->numSM;
   return h->numLists >= 7 * warps ? 0 : h->numLists >= 3 * warps ? 1 : 2;
